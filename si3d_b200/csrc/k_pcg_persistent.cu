@@ -1,4 +1,7 @@
-// Whole CG solve in one cooperative launch.
+// Whole CG solve on both colours in one cooperative launch: the form of stopping test 2, whose norms
+// run over every unknown, and of graphs that are no plain grid or have a handful of nodes; the other
+// solves run on the black unknowns alone (k_pcg_schur.cu, half the vectors and two exchanges an
+// iteration instead of three barriers).
 //
 // The arithmetic of an iteration is that of the three-kernel form in k_zeta.cu (black half of
 // M^-1 fused with u += alpha p and r -= alpha q; red half; p = z + beta p and q = A p on both
@@ -360,25 +363,6 @@ __global__ void __launch_bounds__(PQB, 1) k_pcg_loop(PcgDevT<T> P, GridBar* bar)
   pcg_loop_body<T, TEST2, DIAG>(P, bar, blockIdx.x, gridDim.x);
 }
 
-// The FP64 loops of an ensemble's basins in one cooperative launch: basin m's system is solved by
-// blocks [first, first + nblk) of the grid with its own barrier record, so each basin iterates to
-// its own convergence and the launch ends when the last one has (stopping test 5, no stored
-// diagonal: the basins the ensemble form admits).
-__global__ void __launch_bounds__(PQB, 1) k_pcg_loop_ens(const PcgEnsItem* __restrict__ items, int nitems) {
-  __shared__ PcgEnsItem s_it;
-  __shared__ int s_m;
-  if (threadIdx.x == 0) {
-    int m = -1;
-    for (int i = 0; i < nitems && m < 0; ++i)
-      if ((int)blockIdx.x >= items[i].first && (int)blockIdx.x < items[i].first + items[i].nblk) m = i;
-    s_m = m;
-    if (m >= 0) s_it = items[m];
-  }
-  __syncthreads();
-  if (s_m < 0) return;
-  pcg_loop_body<double, false, false>(s_it.P, s_it.bar, (int)blockIdx.x - s_it.first, s_it.nblk);
-}
-
 // Cooperative launch (all blocks co-resident) through cudaLaunchKernelEx, which stream capture
 // records as a cooperative kernel node.
 template <typename T>
@@ -685,28 +669,6 @@ int pcg_loop_blocks(int device, int nR, int nB, int max_per_sm, bool fp32) {
 
 int pcg_loop(const PcgDev& P, GridBar* bar, int nblocks, bool test2, cudaStream_t st, const GridBar* init) {
   return launch_loop<double>(P, bar, nblocks, test2, st, init);
-}
-
-int pcg_loop_ens_blocks(int device) {
-  int sms = 0, occ = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_pcg_loop_ens, PQB, 0);
-  return sms * std::max(occ, 0);
-}
-
-int pcg_loop_ens(const PcgEnsItem* items, int nitems, int nblocks, GridBar* bars, cudaStream_t st) {
-  if (cudaMemsetAsync(bars, 0, sizeof(GridBar) * (size_t)nitems, st) != cudaSuccess) return -1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nblocks);
-  cfg.blockDim = dim3(PQB);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k_pcg_loop_ens, items, nitems) == cudaSuccess ? 0 : -1;
 }
 
 int pcg_loop_f(const PcgDevF& F, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init) {

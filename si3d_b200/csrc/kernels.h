@@ -36,6 +36,14 @@ struct PcgDevT {
   // the iteration reads the gathered diagonal (matcon's rr) instead of forming it from sx and sy:
   // set for handles with open boundaries, whose cut faces leave rr larger than that sum
   bool diag_stored = false;
+  // the loop on the black unknowns (k_pcg_schur.cu): scratch of the nodes that do not fit in shared
+  // memory (nine coefficients and eight neighbours per black node, and S p), null when the graph's
+  // diagonal neighbours do not close (the two-colour loop runs then); `slots` of its barriers
+  T *cf = nullptr, *sv = nullptr;
+  int* nb8 = nullptr;
+  int reach = 0;              // largest index distance of two coupled black nodes
+  int slot_blocks = 0;        // blocks the slots are laid out for
+  uint4 *slots = nullptr, *zt = nullptr;   // barrier slots; z of every black node as a tagged word
 };
 using PcgDev = PcgDevT<double>;
 using PcgDevF = PcgDevT<float>;
@@ -145,8 +153,17 @@ struct PcgEnsItem {
   int first, nblk;
 };
 int pcg_loop_ens_blocks(int device);   // co-resident blocks of the batched launch
-// the batched launch over nitems basins (items and bars in device memory; bars zeroed first)
-int pcg_loop_ens(const PcgEnsItem* items, int nitems, int nblocks, GridBar* bars, cudaStream_t st);
+// the batched launch over nitems basins (items, bars and slots in device memory; bars and the
+// slot_bytes at slots zeroed first)
+int pcg_loop_ens(const PcgEnsItem* items, int nitems, int nblocks, GridBar* bars, uint4* slots, size_t slot_bytes,
+                 cudaStream_t st);
+// The test-5 loop on the black unknowns (k_pcg_schur.cu).  init: raises the kernels' shared-memory
+// limits; blocks: the launch's grid for nB black nodes; slots: uint4 entries its barriers need.
+int schur_init();
+int schur_blocks(int device, int nB, int max_per_sm);
+size_t schur_slots(int nblocks);
+int schur_loop(const PcgDev& P, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init = nullptr);
+int schur_loop_f(const PcgDevF& F, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init = nullptr);
 int pcg_loop(const PcgDev& P, GridBar* bar, int nblocks, bool test2, cudaStream_t st,
              const GridBar* init = nullptr);   // test2: stopping test 2
 int pcg_loop_f(const PcgDevF& F, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init = nullptr);

@@ -105,7 +105,8 @@ struct Ctx {
   int last_iters = 8;
   // whole-solve cooperative kernel (k_pcg_persistent.cu); false -> one launch per phase
   bool persistent = true;
-  int loop_blocks = 0, loop_blocks_f = 0;   // FP64 / FP32 grids of the cooperative solve
+  int loop_blocks = 0, loop_blocks_f = 0;   // FP64 / FP32 grids of the two-colour cooperative solve
+  int schur_blk = 0;                        // grid of the loop on the black unknowns
   GridBar* bar = nullptr;
   // si3d_gpu_test_wait_limit: barrier record for the next cooperative solve launch only
   GridBar bar_test{};
@@ -597,6 +598,46 @@ int build_pcg(Ctx* c, const si3d_grid* g) {
   if (rc) return rc;
   P.part0 = parts; P.part1 = parts + nblk; P.part2 = parts + 2 * nblk; P.part3 = parts + 3 * nblk;
   P.part_n = nblk;
+  // the loop on the black unknowns (stopping test 5): its rows couple nodes two faces apart, so the
+  // neighbours must close as they do on a plain grid (east of west is the node itself, west of south
+  // is south of west where both exist); other graphs keep the two-colour loop
+  // (a handful of nodes converges exactly, and the rounding that is left then decides between
+  // success and (r, z) = 0: those keep the two-colour loop as well)
+  bool closes = nB >= 32 && c->prm.pcg_test == 5 && c->prm.ordering != SI3D_ORDER_NATURAL &&
+                c->prm.precision != SI3D_MIXED_MG;
+  for (int j = 0; j < nB && closes; ++j) {
+    const int4 q = nbB[j];
+    const int4 none = make_int4(nB, nB, nB, nB);
+    auto red = [&](int k) { return k < nR ? nbR[k] : none; };
+    const int4 kW = red(q.x), kS = red(q.y), kN = red(q.z), kE = red(q.w);
+    auto back = [&](int k, int m) { return k == nR || m == j; };
+    auto meet = [&](int a, int b) { return a == nB || b == nB || a == b; };
+    closes = back(q.x, kW.w) && back(q.y, kS.z) && back(q.z, kN.y) && back(q.w, kE.x) && meet(kW.y, kS.x) &&
+             meet(kW.z, kN.x) && meet(kE.y, kS.w) && meet(kE.z, kN.w);
+    for (const int4& k : {kW, kS, kN, kE})
+      for (int m : {k.x, k.y, k.z, k.w})
+        if (m < nB) P.reach = std::max(P.reach, std::abs(m - j));
+  }
+  c->schur_blk = schur_blocks(c->device, nB, bps ? std::atoi(bps) : 0);
+  if (closes) {
+    const size_t n = std::max(nB, 1);
+    rc |= c->alloc(&P.nb8, 8 * n);
+    rc |= c->alloc(&P.slots, schur_slots(c->schur_blk));
+    rc |= c->alloc(&P.zt, n);
+    if (c->prm.precision == SI3D_MIXED_IR) {
+      rc |= c->alloc(&c->pcgf.cf, 9 * n);
+      rc |= c->alloc(&c->pcgf.sv, n);
+    } else {
+      rc |= c->alloc(&P.cf, 9 * n);
+      rc |= c->alloc(&P.sv, n);
+    }
+    c->pcgf.nb8 = P.nb8;
+    c->pcgf.slots = P.slots;
+    c->pcgf.zt = P.zt;
+    c->pcgf.reach = P.reach;
+    c->pcgf.slot_blocks = P.slot_blocks = c->schur_blk;
+    if (!rc && schur_init() != 0) { g_last_cuda = "zeta-solve shared-memory attribute"; rc = SI3D_ECUDA; }
+  }
   rc |= c->alloc(&P.sc, 1);
   const int cap = std::max(c->prm.pcg_itmax, 1) + 1;
   rc |= c->alloc(&P.hist_alpha, cap);
@@ -779,7 +820,10 @@ int refine(Ctx* c, int* total_inner) {
     CK(cudaMemcpyAsync(c->pcgf.sc, c->h_scf, sizeof(PcgScal), cudaMemcpyHostToDevice, c->st));
     int rci = iterate(c, c->pcgf.sc, c->h_scf, p.pcg_itmax, c->last_inner,
                       [&](int par) { pcg_iteration_f(c->pcgf, par, c->st); },
-                      [&] { return pcg_loop_f(c->pcgf, c->bar, c->loop_blocks_f, c->st, take_bar_test(c)); });
+                      [&] {
+                        return c->pcgf.cf ? schur_loop_f(c->pcgf, c->bar, c->schur_blk, c->st, take_bar_test(c))
+                                          : pcg_loop_f(c->pcgf, c->bar, c->loop_blocks_f, c->st, take_bar_test(c));
+                      });
     if (rci) return rci;
     if (c->h_scf->ier == SI3D_ETIMEOUT) return SI3D_ETIMEOUT;
     const int its = c->h_scf->in;
@@ -881,6 +925,13 @@ int solve_graph_post(Ctx* c, double* hist, int ier) {
   return 0;
 }
 
+// The FP64 MIC-CG loop: on the black unknowns, or on both colours (stopping test 2, whose norms need
+// every unknown, and graphs that are no plain grid).
+int fp64_loop(Ctx* c, const GridBar* init) {
+  if (c->pcg.cf) return schur_loop(c->pcg, c->bar, c->schur_blk, c->st, init);
+  return pcg_loop(c->pcg, c->bar, c->loop_blocks, c->prm.pcg_test == 2, c->st, init);
+}
+
 int solve(Ctx* c, int* iters, double* relres, int* ier_out) {
   const si3d_params& p = c->prm;
   PcgScal init{};
@@ -940,7 +991,7 @@ int solve(Ctx* c, int* iters, double* relres, int* ier_out) {
       c->def_ier = ier;
       return 0;
     }
-    if (pcg_loop(c->pcg, c->bar, c->loop_blocks, c->prm.pcg_test == 2, c->st) != 0) return cuda_fail(cudaGetLastError(), "pcg_loop", __LINE__);
+    if (fp64_loop(c, nullptr) != 0) return cuda_fail(cudaGetLastError(), "pcg_loop", __LINE__);
     c->launches += 1;
     return solve_graph_post(c, hist, ier);
   }
@@ -953,9 +1004,7 @@ int solve(Ctx* c, int* iters, double* relres, int* ier_out) {
     // run iterations in batches; every kernel returns at once after convergence
     int rci = iterate(c, c->pcg.sc, c->h_sc, p.pcg_itmax, c->last_iters,
                       [&](int par) { pcg_iteration(c->pcg, par, c->st); },
-                      [&] {
-                        return pcg_loop(c->pcg, c->bar, c->loop_blocks, c->prm.pcg_test == 2, c->st, take_bar_test(c));
-                      });
+                      [&] { return fp64_loop(c, take_bar_test(c)); });
     if (rci) return rci;
     total_iters = c->h_sc->in;
     c->last_iters = std::max(total_iters, 1);
@@ -1947,6 +1996,8 @@ struct Ens {
   std::vector<int> caps;               // blocks of each member's own solve launch
   PcgEnsItem* d_items = nullptr;       // [slots][members] shares of the batched launches
   GridBar* d_bars = nullptr;
+  uint4* d_slots = nullptr;            // barrier slots of all members, one after the other
+  size_t slot_n = 0;
   ~Ens() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -1955,6 +2006,7 @@ struct Ens {
     if (master) cudaStreamDestroy(master);
     if (d_items) cudaFree(d_items);
     if (d_bars) cudaFree(d_bars);
+    if (d_slots) cudaFree(d_slots);
   }
 };
 std::vector<Ens*> g_ens;
@@ -2002,12 +2054,12 @@ static bool ens_batch_plan(Ens* E) {
   long long own = 0;
   for (int i = 0; i < m; ++i) {
     const Ctx* c = get(E->hs[i]);
-    if (c->prm.pcg_test != 5 || c->pcg.diag_stored || c->rec_buf || c->prm.itrap != p0.itrap ||
-        c->prm.niter != p0.niter || c->loop_blocks < 1)
+    if (!c->pcg.cf || c->pcg.diag_stored || c->rec_buf || c->prm.itrap != p0.itrap ||
+        c->prm.niter != p0.niter || c->schur_blk < 1)
       return false;
-    E->nodes_of[i] = std::max(c->pcg.R.n, c->pcg.B.n);
-    E->caps[i] = c->loop_blocks;
-    own += c->loop_blocks;
+    E->nodes_of[i] = c->pcg.B.n;
+    E->caps[i] = c->schur_blk;
+    own += c->schur_blk;
   }
   const int nb = pcg_loop_ens_blocks(E->device);
   if (nb < m) return false;
@@ -2023,8 +2075,8 @@ static bool ens_batch_plan(Ens* E) {
 // blocks its own launch uses (its partial-sum arrays are sized for those).  Every block of the grid
 // is given out.
 static std::vector<int> ens_shares(const Ens* E, const std::vector<double>& its) {
-  constexpr double kIterUs = 5.0;      // three grid barriers and the partial sums of an iteration
-  constexpr double kNodeUs = 0.0066;   // both colours' streams of one node of the larger colour
+  constexpr double kIterUs = 2.9;      // the two exchanges of an iteration
+  constexpr double kNodeUs = 0.0026;   // one black node (1183 a block: 5.9 us an iteration, 491: 4.1 us)
   const int m = (int)E->hs.size();
   std::vector<int> b(m, 1);
   int left = E->loop_blocks - m;
@@ -2048,12 +2100,15 @@ static std::vector<int> ens_shares(const Ens* E, const std::vector<double>& its)
 static int ens_upload_shares(Ens* E, const std::vector<std::vector<double>>* its) {
   const int m = (int)E->hs.size();
   std::vector<PcgEnsItem> items((size_t)m * E->slots);
+  std::vector<size_t> at(m + 1, 0);
+  for (int i = 0; i < m; ++i) at[i + 1] = at[i] + schur_slots(E->caps[i]);
   for (int k = 0; k < E->slots; ++k) {
     const std::vector<int> b = ens_shares(E, its ? (*its)[k] : std::vector<double>(m, 1.0));
     int first = 0;
     for (int i = 0; i < m; ++i) {
       PcgEnsItem& it = items[(size_t)k * m + i];
       it.P = get(E->hs[i])->pcg;
+      it.P.slots = E->d_slots + at[i];
       it.bar = E->d_bars + i;
       it.first = first;
       it.nblk = b[i];
@@ -2075,6 +2130,8 @@ static int ens_capture_batched(Ens* E) {
   if (!E->d_items) {
     CK(cudaMalloc(&E->d_bars, sizeof(GridBar) * (size_t)m));
     CK(cudaMalloc(&E->d_items, sizeof(PcgEnsItem) * (size_t)m * E->slots));
+    for (int cap : E->caps) E->slot_n += schur_slots(cap);
+    CK(cudaMalloc(&E->d_slots, sizeof(uint4) * E->slot_n));
     const int rc = ens_upload_shares(E, nullptr);
     if (rc) return rc;
   }
@@ -2107,7 +2164,8 @@ static int ens_capture_batched(Ens* E) {
         return cuda_fail(cudaGetLastError());
     }
     if (slot >= E->slots) return SI3D_EDIMS;
-    if (pcg_loop_ens(E->d_items + (size_t)slot * m, m, E->loop_blocks, E->d_bars, E->master) != 0)
+    if (pcg_loop_ens(E->d_items + (size_t)slot * m, m, E->loop_blocks, E->d_bars, E->d_slots,
+                     sizeof(uint4) * E->slot_n, E->master) != 0)
       return cuda_fail(cudaGetLastError(), "pcg_loop_ens", __LINE__);
     ++slot;
     cs[0]->launches += 1;
