@@ -29,6 +29,7 @@ struct Fields3 {
 
 struct Fields2 {
   double *s, *sp, *spp, *eagx, *earx, *eagy, *eary, *sx, *sy, *dd, *qq, *rr, *uair, *vair, *cdw;
+  double *rsx, *rsy;   // sums of 1000 + rhop over the wet layers of the u and v face (momentum)
   int *k1z, *k1u, *k1v;
 };
 
@@ -106,6 +107,11 @@ __device__ __forceinline__ double densty_s(double t, double s, double z) {
 __device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
   const unsigned int s = static_cast<unsigned int>(__cvta_generic_to_shared(smem));
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem) : "memory");
+}
+// 16-byte asynchronous copy (both addresses 16-byte aligned) past the L1, the shared-memory address
+// given as such.
+__device__ __forceinline__ void cp_async16(unsigned int smem, const double* gmem) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(smem), "l"(gmem) : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 template <int N>

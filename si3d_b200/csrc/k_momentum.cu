@@ -10,11 +10,13 @@
 //   interpolation) - and stages them in ag(k) and ar(k), the output arrays of this stage.  A warp
 //   is 32 consecutive face columns at one layer: every field access is a coalesced run of the
 //   layer-major layout, and thousands of independent cells keep the loads in flight.
-// k_mom_columns (one thread per face column): everything that runs down the column - the
-//   depth-mean density, the baroclinic prefix sum, explicit vertical diffusion, the tridiagonal
-//   coefficients and boundary terms (wind and bottom stress) and the Thomas sweeps with two
-//   right-hand sides - reading the staged ex/increment back and writing the final ag/ar.  The c'
-//   coefficients of the forward sweep go to the Thomas scratch array.
+// k_mom_columns (one thread per face column): everything that runs down the column - the baroclinic
+//   prefix sum, explicit vertical diffusion, the tridiagonal coefficients and boundary terms (wind
+//   and bottom stress) and the forward Thomas sweep with two right-hand sides - reading the staged
+//   ex/increment back and writing the eliminated right-hand sides to ag/ar.  The c' coefficients go
+//   to the Thomas scratch array.
+// k_mom_rho sums the density over the depth of both faces of a column first, and k_mom_back runs the
+//   back substitution and sums the depth totals; k_mom_fused is the cell and the column kernel in one.
 // The cell kernel evaluates the reference's expressions in its operation order, except that it
 // multiplies by the reciprocals of the grid constants (4 dx, 4 dy, dx^2, dy^2) where the reference
 // divides by them, and forms the interpolation weights hk / (hk + hkp) as hk * (1 / (hk + hkp)).  The column kernel shares reciprocals between the tridiagonal coefficients (three
@@ -30,6 +32,7 @@ namespace si3d {
 
 namespace {
 
+constexpr int BT = 128;  // threads per block of the streaming kernels
 constexpr int CW = 32;   // face columns per block of the cell kernel (layer lanes per column: CL)
 
 
@@ -230,10 +233,7 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_mom_columns(Dev d, const FaceM
   const double twodt1 = d.p.twodt * d.tz, tz = d.tz, theta = d.p.theta;
   const double gdt = X ? d.p.gdtdx : d.p.gdtdy;
   // depth-mean density (:1277 / :1470)
-  double rsum = 0;
-#pragma unroll 4
-  for (int k = k1x; k <= kmx; ++k) rsum += 1000 + d.f.rhop[IX(d, k, l)];
-  const double rhopx = rsum / nw;
+  const double rhopx = (X ? d.s.rsx : d.s.rsy)[l - 1] / nw;
   const double ws0 = rhopx * gdt * (d.s.spp[lO - 1] - d.s.spp[l - 1]);
   // wind drag coefficient cdw*rhoair*|Uair - usurf| (:1348-1360 / :1540-1552)
   double cwx;
@@ -348,55 +348,124 @@ __global__ void __launch_bounds__(NT, 768 / NT) k_mom_columns(Dev d, const FaceM
     avo = avop; avl = avlp;
     rhkm = rhk; rhk = rhkp; rkm = rkp;
   }
-  // back substitution, summing the depth totals on the way up
-  double d2 = d1p, e2 = e1p;
-  double sg = d2, sr = e2;
-#pragma unroll 4
-  for (int k = kmx - 1; k >= k1x; --k) {
-    const int ik = IX(d, k, l);
-    const double c = cc[ik];
-    d2 = agA[ik] - c * d2;
-    e2 = arA[ik] - c * e2;
-    agA[ik] = d2; arA[ik] = e2;
-    sg += d2; sr += e2;
+}
+
+// ------------------------------------------------------------------ depth sums, back substitution
+// Sum of 1000 + rhop over the wet layers of both faces of a column, in one pass down it (the mean
+// densities of exmom, :1277 / :1470).
+template <int NT>
+__global__ void __launch_bounds__(NT) k_mom_rho(Dev d) {
+  const int l = blockIdx.x * NT + threadIdx.x + 1;
+  if (l > d.g.lm) return;
+  const int lE = NB(d.g.lEC, l), lN = NB(d.g.lNC, l);
+  const int kz = NB(d.g.kmz, l), ku = d.s.k1u[l - 1], kv = d.s.k1v[l - 1];
+  const int kx = min(kz, NB(d.g.kmz, lE)), ky = min(kz, NB(d.g.kmz, lN));
+  double sx = 0, sy = 0;
+#pragma unroll 8
+  for (int k = min(ku, kv); k <= kz; ++k) {
+    const double r = 1000 + d.f.rhop[IX(d, k, l)];
+    if (k >= ku && k <= kx) sx += r;
+    if (k >= kv && k <= ky) sy += r;
   }
+  d.s.rsx[l - 1] = sx;
+  d.s.rsy[l - 1] = sy;
+}
+
+// Back substitution of the momentum systems, summing the depth totals on the way up (one thread per
+// face column).  A kernel of its own because it only streams: with no shared memory it keeps 64 warps
+// and the whole L1 for loads in flight, where the end of the fused kernel (16 warps, a ring that
+// leaves 28 KB of L1) took 0.36 ms a direction at 2000 x 1000 x 60 for five streams.
+template <int IEQ, int NT>
+__global__ void __launch_bounds__(NT) k_mom_back(Dev d, const FaceMeta* __restrict__ meta, int ncols) {
+  const int t = min((int)(blockIdx.x * NT + threadIdx.x), ncols - 1);
+  const bool X = (IEQ == 1);
+  const int l = __ldg(&meta[t].a.x), kmx = __ldg(&meta[t].b.z);
+  const int k1x = NB(X ? d.s.k1u : d.s.k1v, l);
+  const bool act = (int)(blockIdx.x * NT + threadIdx.x) < ncols && k1x <= kmx;
+  double* __restrict__ agA = X ? d.f.agx : d.f.agy;
+  double* __restrict__ arA = X ? d.f.arx : d.f.ary;
+  const double* __restrict__ cc = d.scr;
+  // the lanes of a warp go up together from the deepest of their columns, so that a load is one run
+  // of a layer (each lane starting at its own bottom: 32 layers at once, 0.5 instead of 0.17 ms)
+  const int kw = __reduce_max_sync(0xffffffffu, act ? kmx : 0), kt = __reduce_min_sync(0xffffffffu, act ? k1x : 1 << 20);
+  double d2 = 0, e2 = 0, sg = 0, sr = 0;
+  constexpr int U = 4;   // layers in flight
+  for (int k0 = kw; k0 >= kt; k0 -= U) {
+    double c[U], g[U], r[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 - u, ik = IX(d, k, l);
+      if (act && k >= k1x && k <= kmx) { c[u] = cc[ik]; g[u] = agA[ik]; r[u] = arA[ik]; }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 - u, ik = IX(d, k, l);
+      if (!act || k < k1x || k > kmx) continue;
+      if (k == kmx) {
+        d2 = sg = g[u];
+        e2 = sr = r[u];
+      } else {
+        d2 = g[u] - c[u] * d2;
+        e2 = r[u] - c[u] * e2;
+        agA[ik] = d2; arA[ik] = e2;
+        sg += d2; sr += e2;
+      }
+    }
+  }
+  if (!act) return;
   if (X) { d.s.eagx[l - 1] = sg; d.s.earx[l - 1] = sr; }
   else { d.s.eagy[l - 1] = sg; d.s.eary[l - 1] = sr; }
 }
 
 // ------------------------------------------------------------------ fused kernel
-// k_mom_fused (one thread per face column): the cell and the column work of a face column in one
-// pass down the column.  At layer k the thread forms the explicit term and the baroclinic increment
-// exactly as k_mom_cells does and feeds them straight into the forward sweep of k_mom_columns, so
-// neither goes through memory, and every input is read once.  The values that layer k needs and the
-// layer above it did not (32 FP64 loads: the layer's own cells and its neighbours, and layer k + 1
-// where the sweep or the vertical terms reach down) are copied by cp.async into this thread's slots
-// of a shared-memory ring, RD layers ahead; the values shared with the layer above (thickness,
-// velocity, wp, upp and Av of layer k, depth and density of layer k - 1 for the bottom-layer
-// interpolation) are carried in registers.  Same expressions in the same order as the split
-// kernels: the results are bit-identical to theirs.
+// k_mom_fused (block = one tile of 128 face columns): the cell work and the forward sweep of a face
+// column in one pass down it.  At layer k a thread forms the explicit term and the baroclinic
+// increment of its face exactly as k_mom_cells does and feeds them straight into the forward sweep
+// of k_mom_columns, so neither goes through memory.  The block's columns and their neighbours (at
+// most 2 kMomPairs; a tile is about 4 rows x 32 columns of the grid, so its faces share most of
+// them) are loaded once per field and layer into a shared-memory ring, a pair of columns per 16-byte
+// cp.async, while the layer before is computed; every stencil value is read from there.  A pair is
+// loaded down to the deepest layer that one of its faces reads.  Values of the layer above
+// (thicknesses, velocity, wp, upp, Av of the face) are carried in registers.  Same expressions in the
+// same order as the split kernels: the results are bit-identical to theirs.
+//
+// Bound by instruction issue and the latency of a layer's chain (two divisions) with 16 warps per SM
+// (126 registers, 55 KB of ring).  The form before it had each thread copy its own 32 inputs of a
+// layer, 8 bytes each, and ended with the back substitution: 786 instructions a cell and warp (598
+// now), 8 KB a warp and layer through an L1 that the ring left 28 KB of.  At 2000 x 1000 x 60, per
+// direction with the depth sums and the back substitution: 1.60 and 1.57 ms -> 1.31 and 1.23 ms.
+// Blocks of other sizes, rings of four layers (less L1 for the loads in flight: 1.61 ms), and tiles
+// of 16 columns (1.34 ms: half-filled runs of a layer) were slower.
 namespace fz {
-enum { HKP, HPL, HPO, A0, A1, A2, A3, B0, B1, B2, WDO, WDL, UVD, UVE, UVW, UVN, UVS, OWN, UPP1,
-       HPPL, HPPE, HPPN, HPPW, HPPS, PN, PS, PE, PW, RHO_O, RHO_L, AVO, AVL, NIN };
+enum { HUV, HP, CROSS, ALONG, WP, UV, OWN, UPP, HPP, RHO, AV, NF };   // huv, hp, the other and the own transport, ...
 }
+constexpr int MT = kMomFaces, MU = 2 * kMomPairs;
+constexpr int kMomSlots = 3;   // layers k and k + 1 in use, k + 2 under way
+constexpr int kMomSmem = kMomSlots * fz::NF * MU * (int)sizeof(double);
 
-template <int NT, int RD>
-constexpr int fused_smem() { return RD * fz::NIN * NT * (int)sizeof(double); }
-
-template <int IEQ, int NT, int RD, int MINB>
-__global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* __restrict__ meta, int ncols) {
-  extern __shared__ double ring[];   // [RD][NIN][NT]: a thread's slots are its own
-  const int t = blockIdx.x * NT + threadIdx.x;
-  if (t >= ncols) return;
+template <int IEQ>
+__global__ void __launch_bounds__(MT, 4) k_mom_fused(Dev d, const FaceMeta* __restrict__ meta, MomTiles T) {
+  extern __shared__ double ring[];   // [slot][field][column]
+  __shared__ int s_kmin;
   const bool X = (IEQ == 1);
+  const int tid = threadIdx.x;
+  const int4 tl = __ldg(&T.tile[blockIdx.x]);
+  const int nface = tl.y, npair = tl.w & 0xffff, kmaxb = tl.w >> 16;
+  const bool has = tid < nface;
+  const int t = tl.x + (has ? tid : 0);
   const int4 ma = __ldg(&meta[t].a), mb = __ldg(&meta[t].b);
   const int l = ma.x, lE = ma.y, lW = ma.z, lN = ma.w, lS = mb.x, lX2 = mb.y, kmx = mb.z;
   const int lO = X ? lE : lN;
+  const int mW_last = mb.w, mS_last = __ldg(&meta[t].c.x);
+  // the pair of columns this thread loads, and the last layer that is read of it
+  const int2 cp = tid < npair ? __ldg(&T.pair[tl.z + tid]) : make_int2(0, 0);
+  if (tid == 0) s_kmin = 1 << 20;
   const int* k1f = X ? d.s.k1u : d.s.k1v;
   const int k1x = NB(k1f, l);
   const int nw = kmx - k1x + 1;
-  if (nw < 1) return;
-  const int mW_last = mb.w, mS_last = __ldg(&meta[t].c.x);
+  const bool act = has && nw >= 1;
+  __syncthreads();
+  if (act) atomicMin(&s_kmin, k1x);
   const int mW_first = mW_last >= 0 ? NB(k1f, lW) : 0;
   const int mS_first = mS_last >= 0 ? NB(k1f, lS) : 0;
   const double* __restrict__ huv = X ? d.f.hup : d.f.hvp;
@@ -404,8 +473,8 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
   const double* __restrict__ uvpp_h = X ? d.f.uhpp : d.f.vhpp;
   const double* __restrict__ uvp = X ? d.f.up : d.f.vp;
   const double* __restrict__ uvpp = X ? d.f.upp : d.f.vpp;
-  const double* __restrict__ vhp = d.f.vhp;
-  const double* __restrict__ uhp = d.f.uhp;
+  const double* __restrict__ cross = X ? d.f.vhp : d.f.uhp;
+  const double* __restrict__ along = X ? d.f.uhp : d.f.vhp;
   const double* __restrict__ wp = d.f.wp;
   const double* __restrict__ hp3 = d.f.hp;
   const double* __restrict__ rhop = d.f.rhop;
@@ -417,68 +486,38 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
   const double gdt = X ? d.p.gdtdx : d.p.gdtdy;
   const bool ihd = d.p.ihd == 1, ibc = d.p.ibc != 0;
   const int P = d.g.P;
-  const int dE = lE - l, dW = lW - l, dN = lN - l, dS = lS - l, dX2 = lX2 - l, dO = lO - l;
-  const int tid = threadIdx.x;
-  auto sp = [&](int s, int i) { return &ring[(s * fz::NIN + i) * NT + tid]; };
-  auto issue = [&](int kk, int s) {   // the new inputs of layer kk into ring slot s
-    const int ikk = IX(d, kk, l);
-    cp_async8(sp(s, fz::HKP), &huv[ikk + P]);
-    cp_async8(sp(s, fz::HPL), &hp3[ikk]);
-    cp_async8(sp(s, fz::HPO), &hp3[ikk + dO]);
-    if (X) {
-      cp_async8(sp(s, fz::A0), &vhp[ikk + dE]);
-      cp_async8(sp(s, fz::A1), &vhp[ikk]);
-      cp_async8(sp(s, fz::A2), &vhp[ikk + dX2]);
-      cp_async8(sp(s, fz::A3), &vhp[ikk + dS]);
-      cp_async8(sp(s, fz::B0), &uhp[ikk + dE]);
-      cp_async8(sp(s, fz::B1), &uhp[ikk]);
-      cp_async8(sp(s, fz::B2), &uhp[ikk + dW]);
-    } else {
-      cp_async8(sp(s, fz::A0), &uhp[ikk + dN]);
-      cp_async8(sp(s, fz::A1), &uhp[ikk]);
-      cp_async8(sp(s, fz::A2), &uhp[ikk + dX2]);
-      cp_async8(sp(s, fz::A3), &uhp[ikk + dW]);
-      cp_async8(sp(s, fz::B0), &vhp[ikk + dN]);
-      cp_async8(sp(s, fz::B1), &vhp[ikk]);
-      cp_async8(sp(s, fz::B2), &vhp[ikk + dS]);
-    }
-    cp_async8(sp(s, fz::WDO), &wp[ikk + P + dO]);
-    cp_async8(sp(s, fz::WDL), &wp[ikk + P]);
-    cp_async8(sp(s, fz::UVD), &uvp[ikk + P]);
-    cp_async8(sp(s, fz::UVE), &uvp[ikk + dE]);
-    cp_async8(sp(s, fz::UVW), &uvp[ikk + dW]);
-    cp_async8(sp(s, fz::UVN), &uvp[ikk + dN]);
-    cp_async8(sp(s, fz::UVS), &uvp[ikk + dS]);
-    cp_async8(sp(s, fz::OWN), &uvpp_h[ikk]);
-    cp_async8(sp(s, fz::UPP1), &uvpp[ikk + P]);
-    if (ihd) {
-      cp_async8(sp(s, fz::HPPL), &huvpp[ikk]);
-      cp_async8(sp(s, fz::HPPE), &huvpp[ikk + dE]);
-      cp_async8(sp(s, fz::HPPN), &huvpp[ikk + dN]);
-      cp_async8(sp(s, fz::HPPW), &huvpp[ikk + dW]);
-      cp_async8(sp(s, fz::HPPS), &huvpp[ikk + dS]);
-      cp_async8(sp(s, fz::PN), &uvpp[ikk + dN]);
-      cp_async8(sp(s, fz::PS), &uvpp[ikk + dS]);
-      cp_async8(sp(s, fz::PE), &uvpp[ikk + dE]);
-      cp_async8(sp(s, fz::PW), &uvpp[ikk + dW]);
-    }
-    if (ibc) {
-      cp_async8(sp(s, fz::RHO_O), &rhop[ikk + dO]);
-      cp_async8(sp(s, fz::RHO_L), &rhop[ikk]);
-    }
-    cp_async8(sp(s, fz::AVO), &Av[ikk + P + dO]);
-    cp_async8(sp(s, fz::AVL), &Av[ikk + P]);
+  const int dO = lO - l;
+  // this thread's stencil columns in the ring
+  const uint2 pk = __ldg(&T.idx[t]);
+  const int iC = pk.x & 255, iE = pk.x >> 8 & 255, iW = pk.x >> 16 & 255, iN = pk.x >> 24, iS = pk.y & 255, iX2 = pk.y >> 8 & 255;
+  const int iO = X ? iE : iN;
+  const unsigned int ring0 = static_cast<unsigned int>(__cvta_generic_to_shared(&ring[2 * tid]));
+  __syncthreads();
+  const int kmin = s_kmin;
+  auto issue = [&](int k, int slot) {   // layer k of this thread's pair of columns into ring slot `slot`
+    if (k > cp.y) return;
+    const unsigned int sm = ring0 + (unsigned int)(slot * fz::NF * MU * (int)sizeof(double));
+    const int i = (k - 1) * P + cp.x;
+    auto put = [&](int f, const double* g) { cp_async16(sm + (unsigned int)(f * MU * (int)sizeof(double)), g + i); };
+    put(fz::HUV, huv);
+    put(fz::HP, hp3);
+    put(fz::CROSS, cross);
+    put(fz::ALONG, along);
+    put(fz::WP, wp);
+    put(fz::UV, uvp);
+    put(fz::OWN, uvpp_h);
+    put(fz::UPP, uvpp);
+    if (ihd) put(fz::HPP, huvpp);
+    if (ibc) put(fz::RHO, rhop);
+    put(fz::AV, Av);
   };
-#pragma unroll
-  for (int j = 0; j < RD; ++j) {   // one commit group per layer (empty past the bottom)
-    if (k1x + j <= kmx) issue(k1x + j, j);
-    cp_async_commit();
+  if (kmin <= kmaxb) {
+    issue(kmin, 0);
+    issue(kmin + 1, 1);
   }
+  cp_async_commit();
   // column totals and surface / bottom terms while the first layers are in flight (as k_mom_columns)
-  double rsum = 0;
-#pragma unroll 4
-  for (int k = k1x; k <= kmx; ++k) rsum += 1000 + rhop[IX(d, k, l)];
-  const double rhopx = rsum / nw;
+  const double rhopx = (X ? d.s.rsx : d.s.rsy)[l - 1] / nw;
   const double ws0 = rhopx * gdt * (d.s.spp[lO - 1] - d.s.spp[l - 1]);
   double cwx;
   {
@@ -513,47 +552,83 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
   double hkm = huv[ik0 - P], hk = huv[ik0];
   double upm = uvpp[ik0 - P], upk = uvpp[ik0];
   double uvU = uvp[ik0 - P], uc = uvp[ik0];
-  double avo = Av[ik0 + dO], avl = Av[ik0];
-  double wprev = 0.0;                                       // wp sum of layer k (the layer above's wD)
+  double avo = 0.0, avl = 0.0;                              // no exchange through the surface
+  double wprev = 0.0;                                       // wp sum of layer k (the layer above's wD); none at the surface
   double thq_prev = 0.0;                                    // hkm / (hkm + hk) of layer k
-  double hpl_prev = 0.0, hpo_prev = 0.0, ro_prev = 0.0, rl_prev = 0.0;
   const double rrho = 1.0 / rhopx;
   double rhk = 1.0 / hk, rhkm = 0.0, rkm = 0.0;
   double bcl = 0, c1p = 0, d1p = 0, e1p = 0, hdr_prev = 0;
-  for (int k = k1x, s = 0; k <= kmx; ++k, s = (s + 1 == RD) ? 0 : s + 1) {
+  // baroclinic increment of the bottom layer (bclnc_km), for all columns of the warp at once: inside
+  // the layer loop it would run once for every depth among them
+  double hdr_bot = 0.0;
+  bool bot = false;
+  if (ibc && kmx > k1x) {
+    const int ib = IX(d, kmx, l), io = ib + dO;
+    const double hb = huv[ib];
+    const double hpo = hp3[io], hpl = hp3[ib], hpo_u = hp3[io - P], hpl_u = hp3[ib - P];
+    const double ro = rhop[io], rl = rhop[ib], ro_u = rhop[io - P], rl_u = rhop[ib - P];
+    const double eps = 2.220446049250313e-16;
+    const double hplus = hb + eps, hminus = hb - eps;
+    const bool co = hpo > hplus || hpo < hminus, cw = hpl > hplus || hpl < hminus;
+    double rho_o = ro, rho_w = rl;
+    if (co) {
+      const double dz1 = 0.5 * (hpo_u + hpo);
+      const double dz2 = 0.5 * (hpo_u + hb);
+      rho_o = ro_u + (dz2 / dz1) * (ro - ro_u);
+    }
+    if (cw) {
+      const double dz1 = 0.5 * (hpl_u + hpl);
+      const double dz2 = 0.5 * (hpl_u + hb);
+      rho_w = rl_u + (dz2 / dz1) * (rl - rl_u);
+    }
+    bot = co || cw;
+    hdr_bot = gdt * hb * (rho_o - rho_w);
+  }
+  int s0 = 0, s1 = 1, s2 = 2;   // ring slots of layers k, k + 1, k + 2
+  for (int k = kmin; k <= kmaxb; ++k) {
+    cp_async_wait<0>();   // layers k and k + 1 have landed: this thread's copies, then everyone's
+    __syncthreads();      // (and everyone has left layer k - 1, whose slot is filled next)
+    if (k < kmaxb) issue(k + 2, s2);
+    cp_async_commit();
+    const double* const rk = ring + s0 * fz::NF * MU;   // layer k
+    const double* const rd = ring + s1 * fz::NF * MU;   // layer k + 1
+    { const int q = s0; s0 = s1; s1 = s2; s2 = q; }
+    if (!act || k < k1x || k > kmx) continue;
     const int ik = IX(d, k, l);
-    cp_async_wait<RD - 1>();   // layer k's group has landed (this thread's own copies)
-    const double hkp = *sp(s, fz::HKP);
-    const double hpl = *sp(s, fz::HPL), hpo = *sp(s, fz::HPO);
+    auto at = [&](int f, int i) { return rk[f * MU + i]; };
+    auto below = [&](int f, int i) { return rd[f * MU + i]; };
+    const double hkp = below(fz::HUV, iC);
+    const double hpl = at(fz::HP, iC), hpo = at(fz::HP, iO);
     // ---- explicit term (k_mom_cells)
     double cor, uE, uW, vN, vS;
     if (X) {
-      const double vE = *sp(s, fz::A0), vC = *sp(s, fz::A1), vX = *sp(s, fz::A2), vSS = *sp(s, fz::A3);
-      const double uEE = *sp(s, fz::B0), uC = *sp(s, fz::B1), uWW = *sp(s, fz::B2);
+      const double vE = at(fz::CROSS, iE), vC = at(fz::CROSS, iC), vX = at(fz::CROSS, iX2), vSS = at(fz::CROSS, iS);
+      const double uEE = at(fz::ALONG, iE), uC = at(fz::ALONG, iC), uWW = at(fz::ALONG, iW);
       cor = 0.25 * d.p.f * (vE + vC + vX + vSS);
       uE = uEE + uC;
       uW = uC + uWW;
       vN = vE + vC;
       vS = vX + vSS;
     } else {
-      const double uN = *sp(s, fz::A0), uC = *sp(s, fz::A1), uX = *sp(s, fz::A2), uWW = *sp(s, fz::A3);
-      const double vNN = *sp(s, fz::B0), vC = *sp(s, fz::B1), vSS = *sp(s, fz::B2);
+      const double uN = at(fz::CROSS, iN), uC = at(fz::CROSS, iC), uX = at(fz::CROSS, iX2), uWW = at(fz::CROSS, iW);
+      const double vNN = at(fz::ALONG, iN), vC = at(fz::ALONG, iC), vSS = at(fz::ALONG, iS);
       cor = 0.25 * d.p.f * (uN + uC + uX + uWW);
       uE = uN + uC;
       uW = uX + uWW;
       vN = vNN + vC;
       vS = vC + vSS;
     }
-    const double wDraw = *sp(s, fz::WDO) + *sp(s, fz::WDL);
-    double wU = wprev, wD = wDraw;
-    const double uvD = *sp(s, fz::UVD);
-    const double uvE = *sp(s, fz::UVE), uvW = *sp(s, fz::UVW), uvN = *sp(s, fz::UVN), uvS = *sp(s, fz::UVS);
-    const double own_pp = *sp(s, fz::OWN);
+    const double wDraw = below(fz::WP, iO) + below(fz::WP, iC);
+    const double wU = wprev;
+    double wD = wDraw;
+    const double uvD = below(fz::UV, iC);
+    const double uvE = at(fz::UV, iE), uvW = at(fz::UV, iW), uvN = at(fz::UV, iN), uvS = at(fz::UV, iS);
+    const double own_pp = at(fz::OWN, iC);
     double hd = 0.0;
     if (ihd) {
-      const double hppl = *sp(s, fz::HPPL), hppE = *sp(s, fz::HPPE), hppN = *sp(s, fz::HPPN);
-      const double hppW = *sp(s, fz::HPPW), hppS = *sp(s, fz::HPPS);
-      const double pc = upk, pN = *sp(s, fz::PN), pS = *sp(s, fz::PS), pE = *sp(s, fz::PE), pW = *sp(s, fz::PW);
+      const double hppl = at(fz::HPP, iC), hppE = at(fz::HPP, iE), hppN = at(fz::HPP, iN);
+      const double hppW = at(fz::HPP, iW), hppS = at(fz::HPP, iS);
+      const double pc = upk, pN = at(fz::UPP, iN), pS = at(fz::UPP, iS), pE = at(fz::UPP, iE), pW = at(fz::UPP, iW);
       const double ax_l = d.p.Ax0 * fmin(hppE, hppl);
       const double ay_l = d.p.Ay0 * fmin(hppN, hppl);
       const double ax_w = face_coef(d, d.p.Ax0, hppl, hppW, lW, mW_first, mW_last, k);
@@ -568,11 +643,9 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
     if (hpl <= ZERO || hpo <= ZERO) {
       ex = own_pp;
     } else {
-      const double th_k = (k == k1x) ? 0.0 : thq_prev;
-      const double th1_k = (k == k1x) ? 0.0 : 1. - th_k;
-      const double th_kp = (k == kmx) ? 0.5 : thq;
-      const double th1_kp = (k == kmx) ? 0.5 : 1. - th_kp;
-      if (k == k1x) wU = 0.0;
+      // (the weights at the surface and the bottom, where the reference sets its own, meet a zero wU, wD)
+      const double th_k = thq_prev, th1_k = 1. - th_k;
+      const double th_kp = thq, th1_kp = 1. - th_kp;
       if (k == kmx) wD = 0.0;
       const double scE = uvE + uc, scW = uvW + uc;
       const double scN = uvN + uc, scS = uvS + uc;
@@ -581,52 +654,24 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
       if (X) ex = own_pp - twodt1 * (adv * d.p.iadv - cor - hd);
       else ex = own_pp - twodt1 * (adv * d.p.iadv + cor - hd);
     }
-    // ---- baroclinic increment, bottom layer via bclnc_km (layer k - 1 carried)
-    double hdr = 0, ro = 0, rl = 0;
+    // ---- baroclinic increment
+    double hdr = 0;
     if (ibc) {
-      ro = *sp(s, fz::RHO_O);
-      rl = *sp(s, fz::RHO_L);
-      hdr = gdt * hk * (ro - rl);
-      if (k == kmx && kmx > k1x) {
-        const double eps = 2.220446049250313e-16;
-        const double hplus = hk + eps, hminus = hk - eps;
-        bool co, cw;
-        double rho_o, rho_w;
-        if (hpo > hplus || hpo < hminus) {
-          co = true;
-          const double dz1 = 0.5 * (hpo_prev + hpo);
-          const double dz2 = 0.5 * (hpo_prev + hk);
-          rho_o = ro_prev + (dz2 / dz1) * (ro - ro_prev);
-        } else { co = false; rho_o = ro; }
-        if (hpl > hplus || hpl < hminus) {
-          cw = true;
-          const double dz1 = 0.5 * (hpl_prev + hpl);
-          const double dz2 = 0.5 * (hpl_prev + hk);
-          rho_w = rl_prev + (dz2 / dz1) * (rl - rl_prev);
-        } else { cw = false; rho_w = rl; }
-        if (co || cw) hdr = gdt * hk * (rho_o - rho_w);
-      }
+      hdr = gdt * hk * (at(fz::RHO, iO) - at(fz::RHO, iC));
+      if (k == kmx && bot) hdr = hdr_bot;
     }
     // ---- forward sweep (k_mom_columns)
-    const double upp1 = *sp(s, fz::UPP1);
-    const double avop = *sp(s, fz::AVO), avlp = *sp(s, fz::AVL);
+    const double upp1 = below(fz::UPP, iC);
+    const double avop = below(fz::AV, iO), avlp = below(fz::AV, iC);
     const double rhkp = 1.0 / hkp;
-    const double Avk = (k > k1x) ? 0.5 * (avo + avl) : 0.0;
+    const double Avk = 0.5 * (avo + avl);   // zero at the surface
     const double Avkp = (k < kmx) ? 0.5 * (avop + avlp) : 0.0;
-    double vdiff = 0.0;
-    if (nw >= 2) {
-      const double fk = (k > k1x) ? Avk * (upm - upk) * rkm : 0.0;
-      const double fkp = (k < kmx) ? Avkp * (upk - upp1) * rkp : 0.0;
-      vdiff = d.p.twodt * (fk - fkp) * 2. * (1. - theta);
-    }
-    double a1 = 0, a2, a3 = 0;
-    if (nw == 1) {
-      a2 = 1.0;
-    } else {
-      if (k < kmx) a3 = -twodt1 * Avkp * (rhkp * rkp) * 2. * theta;
-      if (k > k1x) a1 = -twodt1 * Avk * (rhkm * rkm) * 2. * theta;
-      a2 = 1.0 - (hkm * rhk) * a1 - (hkp * rhk) * a3;
-    }
+    const double vdiff = d.p.twodt * (Avk * (upm - upk) * rkm - Avkp * (upk - upp1) * rkp) * 2. * (1. - theta);
+    // (below the bottom layer 1 / hkp is infinite)
+    const double a1 = -twodt1 * Avk * (rhkm * rkm) * 2. * theta;
+    const double a3 = (k < kmx) ? -twodt1 * Avkp * (rhkp * rkp) * 2. * theta : 0.0;
+    double a2 = 1.0;
+    if (nw > 1) a2 = 1.0 - (hkm * rhk) * a1 - (hkp * rhk) * a3;
     if (ibc) {
       if (k == k1x) bcl = hdr;
       else if (X) { const double aaux = hdr_prev + hdr; bcl = bcl + aaux; }
@@ -649,9 +694,6 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
       e1v = (hh - a1 * e1p) * r;
     }
     cc[ik] = c1v; agA[ik] = d1v; arA[ik] = e1v;
-    // refill the slot with layer k + RD (its values are consumed: the stores above depend on them)
-    if (k + RD <= kmx) issue(k + RD, s);
-    cp_async_commit();
     c1p = c1v; d1p = d1v; e1p = e1v;
     hkm = hk; hk = hkp;
     upm = upk; upk = upp1;
@@ -660,57 +702,25 @@ __global__ void __launch_bounds__(NT, MINB) k_mom_fused(Dev d, const FaceMeta* _
     uvU = uc; uc = uvD;
     wprev = wDraw;
     thq_prev = thq;
-    hpl_prev = hpl; hpo_prev = hpo; ro_prev = ro; rl_prev = rl;
   }
-  // back substitution, summing the depth totals on the way up
-  double d2 = d1p, e2 = e1p;
-  double sg = d2, sr = e2;
-#pragma unroll 4
-  for (int k = kmx - 1; k >= k1x; --k) {
-    const int ik = IX(d, k, l);
-    const double c = cc[ik];
-    d2 = agA[ik] - c * d2;
-    e2 = arA[ik] - c * e2;
-    agA[ik] = d2; arA[ik] = e2;
-    sg += d2; sr += e2;
-  }
-  if (X) { d.s.eagx[l - 1] = sg; d.s.earx[l - 1] = sr; }
-  else { d.s.eagy[l - 1] = sg; d.s.eary[l - 1] = sr; }
-}
-
-// MINB: resident blocks per SM the register budget is sized for (the ring's shared memory allows
-// 7 blocks of 64 threads, 3 of 128, 1 of 256)
-template <int IEQ, int NT, int RD, int MINB>
-void launch_fused(const Dev& d, const FaceMeta* cols, int ncols, cudaStream_t st) {
-  k_mom_fused<IEQ, NT, RD, MINB><<<(ncols + NT - 1) / NT, NT, fused_smem<NT, RD>(), st>>>(d, cols, ncols);
-}
-
-template <int NT, int RD, int MINB>
-int fused_attr() {
-  const int b = fused_smem<NT, RD>();
-  if (cudaFuncSetAttribute(k_mom_fused<1, NT, RD, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, b) != cudaSuccess ||
-      cudaFuncSetAttribute(k_mom_fused<2, NT, RD, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, b) != cudaSuccess)
-    return -1;
-  return 0;
 }
 
 }  // namespace
 
 int momentum_init(int km1) {
-  (void)km1;   // the fused kernel's ring is sized by its threads, not by the column depth
-  if (fused_attr<64, 2, 7>() || fused_attr<128, 2, 3>() || fused_attr<256, 2, 1>()) return -1;
+  (void)km1;   // the fused kernel's ring does not depend on the column depth
+  if (cudaFuncSetAttribute(k_mom_fused<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMomSmem) != cudaSuccess ||
+      cudaFuncSetAttribute(k_mom_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMomSmem) != cudaSuccess)
+    return -1;
   return 0;
 }
 
 template <int IEQ>
-void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const Tune& tu, cudaStream_t st, const ObcDev* obc,
-                int nobc) {
+void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu, cudaStream_t st,
+                const ObcDev* obc, int nobc) {
   if (tu.mom_cl == 1 && nobc == 0) {   // one pass per column (open boundaries need the split kernels)
-    switch (tu.mom_nt) {
-      case 64: launch_fused<IEQ, 64, 2, 7>(d, cols, ncols, st); break;
-      case 256: launch_fused<IEQ, 256, 2, 1>(d, cols, ncols, st); break;
-      default: launch_fused<IEQ, 128, 2, 3>(d, cols, ncols, st); break;
-    }
+    k_mom_fused<IEQ><<<tiles.ntile, MT, kMomSmem, st>>>(d, cols, tiles);
+    k_mom_back<IEQ, BT><<<(ncols + BT - 1) / BT, BT, 0, st>>>(d, cols, ncols);
     return;
   }
   const int g1 = (ncols + CW - 1) / CW;
@@ -726,13 +736,15 @@ void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const Tune& tu, c
     case 256: k_mom_columns<IEQ, 256><<<(ncols + 255) / 256, 256, 0, st>>>(d, cols, ncols); break;
     default: k_mom_columns<IEQ, 128><<<(ncols + 127) / 128, 128, 0, st>>>(d, cols, ncols); break;
   }
+  k_mom_back<IEQ, BT><<<(ncols + BT - 1) / BT, BT, 0, st>>>(d, cols, ncols);
 }
 
-void launch_momentum(const Dev& d, int ieq, const FaceMeta* cols, int ncols, const Tune& tu, cudaStream_t st,
-                     const ObcDev* obc, int nobc) {
+void launch_momentum(const Dev& d, int ieq, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu,
+                     cudaStream_t st, const ObcDev* obc, int nobc) {
+  if (ieq == 1) k_mom_rho<BT><<<(d.g.lm + BT - 1) / BT, BT, 0, st>>>(d);   // both directions' sums
   if (ncols <= 0) return;
-  if (ieq == 1) launch_dir<1>(d, cols, ncols, tu, st, obc, nobc);
-  else launch_dir<2>(d, cols, ncols, tu, st, obc, nobc);
+  if (ieq == 1) launch_dir<1>(d, cols, ncols, tiles, tu, st, obc, nobc);
+  else launch_dir<2>(d, cols, ncols, tiles, tu, st, obc, nobc);
 }
 
 }  // namespace si3d

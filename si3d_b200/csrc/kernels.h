@@ -49,10 +49,10 @@ using PcgDev = PcgDevT<double>;
 using PcgDevF = PcgDevT<float>;
 
 // Launch shapes of the column stages that the autotuner picks per handle (results do not depend on
-// them): layer lanes per column of the cell-parallel kernels (2, 4, 8) and threads per block of the
-// column-sequential kernels (64, 128, 256).
+// them): layer lanes per column of the cell-parallel kernels (2, 4, 8; momentum 1: the fused kernel)
+// and threads per block of the column-sequential kernels (64, 128, 256).
 struct Tune {
-  int mom_cl = 8, mom_nt = 128, sal_cl = 8, sal_nt = 128;
+  int mom_cl = 1, mom_nt = 128, sal_cl = 8, sal_nt = 128;
 };
 
 // Static indices of one u (v) face column of the momentum stage, computed once from the grid maps
@@ -64,14 +64,27 @@ struct FaceMeta {
   int4 a, b, c;
 };
 
+// The face columns of the fused momentum kernel in tiles of at most kMomFaces faces that read at most
+// kMomPairs distinct column pairs (columns 2q + 1 and 2q + 2: 16 aligned bytes of a layer).  tile =
+// (first face, faces, first entry of pair, pairs | deepest face layer << 16); pair = (element 2q of
+// a layer, last layer that a face of the tile reads of it), ascending; idx = a face's columns l, lE,
+// lW, lN, lS, lX2 as positions among its tile's columns, 8 bits each.
+constexpr int kMomFaces = 128, kMomPairs = 104;
+struct MomTiles {
+  const int4* tile = nullptr;
+  const int2* pair = nullptr;
+  const uint2* idx = nullptr;
+  int ntile = 0;
+};
+
 int momentum_init(int km1);
 // Raises the continuity kernels' shared-memory limit for columns deeper than 95 levels.
 int transport_init(int km1);
 struct ObcDev;
 // `obc` (nobc boundaries): open boundaries whose face columns' explicit term is recomputed between
 // the cell and the column kernels
-void launch_momentum(const Dev& d, int ieq, const FaceMeta* meta, int ncols, const Tune& tu, cudaStream_t st,
-                     const ObcDev* obc = nullptr, int nobc = 0);
+void launch_momentum(const Dev& d, int ieq, const FaceMeta* meta, int ncols, const MomTiles& tiles, const Tune& tu,
+                     cudaStream_t st, const ObcDev* obc = nullptr, int nobc = 0);
 void launch_matcon(const Dev& d, cudaStream_t st);
 
 void pcg_setup(const Dev& d, const PcgDev& P, int x0_mode, const double* dz, const double* hist, int* negpiv,

@@ -11,6 +11,7 @@
 #include <memory>
 #include <mutex>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/si3d_gpu.h"
@@ -83,6 +84,7 @@ struct Ctx {
   int nce = 0, ncn = 0;
   FaceMeta* mce = nullptr;   // static indices of the u / v face columns (momentum stage)
   FaceMeta* mcn = nullptr;
+  MomTiles tce, tcn;         // their tiles (fused momentum kernel)
   // red-black zeta system
   PcgDev pcg{};
   PcgDevF pcgf{};            // FP32 inner system of iterative refinement
@@ -385,6 +387,61 @@ void colour_columns(int lm, const int* lEC, const int* lWC, const int* lNC, cons
       }
     }
   }
+}
+
+// Tiles of the fused momentum kernel: faces are taken in order until a tile is full, or its pairs of
+// columns are.
+int build_tiles(Ctx* c, const std::vector<FaceMeta>& m, MomTiles* T) {
+  std::vector<int4> tile;
+  std::vector<int2> pair;
+  std::vector<uint2> idx(m.size());
+  std::vector<int> pos(c->lm1 / 2 + 1, -1);   // a pair's entry in the open tile, -1 outside it
+  std::vector<int> q, last, order, place;
+  for (size_t f = 0; f < m.size();) {
+    const size_t first = f;
+    int kmax = 0;
+    q.clear();
+    last.clear();
+    for (; f < m.size() && f - first < (size_t)kMomFaces; ++f) {
+      int p[6] = {m[f].a.x, m[f].a.y, m[f].a.z, m[f].a.w, m[f].b.x, m[f].b.y}, fresh = 0;
+      for (int i = 0; i < 6; ++i) {
+        p[i] = (p[i] - 1) / 2;
+        fresh += pos[p[i]] < 0 && std::find(p, p + i, p[i]) == p + i;
+      }
+      if ((int)q.size() + fresh > kMomPairs) break;
+      const int kmx = m[f].b.z;
+      for (int v : p) {
+        if (pos[v] < 0) { pos[v] = (int)q.size(); q.push_back(v); last.push_back(0); }
+        last[pos[v]] = std::max(last[pos[v]], kmx + 1);   // the sweep reaches one layer below the face
+      }
+      kmax = std::max(kmax, kmx);
+    }
+    // ascending: consecutive threads load consecutive addresses
+    order.resize(q.size());
+    place.resize(q.size());
+    for (size_t i = 0; i < order.size(); ++i) order[i] = (int)i;
+    std::sort(order.begin(), order.end(), [&](int a, int b) { return q[a] < q[b]; });
+    for (size_t i = 0; i < order.size(); ++i) place[order[i]] = (int)i;
+    tile.push_back(make_int4((int)first, (int)(f - first), (int)pair.size(), (int)q.size() | kmax << 16));
+    for (int o : order) pair.push_back(make_int2(2 * q[o], last[o]));
+    for (size_t k = first; k < f; ++k) {
+      auto at = [&](int v) { return (unsigned int)(2 * place[pos[(v - 1) / 2]] + ((v - 1) & 1)); };
+      idx[k].x = at(m[k].a.x) | at(m[k].a.y) << 8 | at(m[k].a.z) << 16 | at(m[k].a.w) << 24;
+      idx[k].y = at(m[k].b.x) | at(m[k].b.y) << 8;
+    }
+    for (int v : q) pos[v] = -1;
+  }
+  int4* dt = nullptr;
+  int2* dp = nullptr;
+  uint2* di = nullptr;
+  if (c->alloc(&dt, tile.size()) || c->alloc(&dp, pair.size()) || c->alloc(&di, idx.size())) return SI3D_ENOMEM;
+  if (!tile.empty()) {
+    CK(cudaMemcpy(dt, tile.data(), tile.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(dp, pair.data(), pair.size() * sizeof(int2), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(di, idx.data(), idx.size() * sizeof(uint2), cudaMemcpyHostToDevice));
+  }
+  *T = MomTiles{dt, dp, di, (int)tile.size()};
+  return 0;
 }
 
 // Aggregation hierarchy of the MG inner solves.  Level 0 is the (im1, jm1) image of the wet
@@ -1061,8 +1118,8 @@ int obc_uvh(Ctx* c) {
 
 // Stages with the open-boundary adjustments that follow their kernels.
 void momentum_stage(Ctx* c, int ieq) {
-  if (ieq == 1) launch_momentum(c->d, 1, c->mce, c->nce, c->tune, c->st, c->obc.data(), (int)c->obc.size());
-  else launch_momentum(c->d, 2, c->mcn, c->ncn, c->tune, c->st, c->obc.data(), (int)c->obc.size());
+  if (ieq == 1) launch_momentum(c->d, 1, c->mce, c->nce, c->tce, c->tune, c->st, c->obc.data(), (int)c->obc.size());
+  else launch_momentum(c->d, 2, c->mcn, c->ncn, c->tcn, c->tune, c->st, c->obc.data(), (int)c->obc.size());
 }
 void matcon_stage(Ctx* c) {
   launch_matcon(c->d, c->st);
@@ -1100,8 +1157,8 @@ int fd_pre(Ctx* c, int istep) {
   if (rc) return rc;
   c->launches += obc_launches(c);
   // surfbc CASE(0) is a constant per-column wind set by the host (uair/vair/cdw fields)
-  rc = stage(c, ST_MOMX, 2 + obc_launches(c), [&] { momentum_stage(c, 1); });
-  if (!rc) rc = stage(c, ST_MOMY, 2 + obc_launches(c), [&] { momentum_stage(c, 2); });
+  rc = stage(c, ST_MOMX, 4 + obc_launches(c), [&] { momentum_stage(c, 1); });
+  if (!rc) rc = stage(c, ST_MOMY, 3 + obc_launches(c), [&] { momentum_stage(c, 2); });
   if (!rc) rc = stage(c, ST_MATCON, 1 + 2 * obc_launches(c), [&] { matcon_stage(c); });
   return rc;
 }
@@ -1276,7 +1333,7 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
     rc |= c->alloc(q, n3);
   Fields2& s = d.s;
   for (double** q : {&s.s, &s.sp, &s.spp, &s.eagx, &s.earx, &s.eagy, &s.eary, &s.sx, &s.sy, &s.dd, &s.qq, &s.rr,
-                     &s.uair, &s.vair, &s.cdw})
+                     &s.uair, &s.vair, &s.cdw, &s.rsx, &s.rsy})
     rc |= c->alloc(q, P);
   for (int** q : {&s.k1z, &s.k1u, &s.k1v}) rc |= c->alloc(q, P);
   rc |= c->alloc(&d.scr, n3);
@@ -1368,13 +1425,29 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
       return m;
     };
     std::vector<FaceMeta> me, mn;
-    for (int l : ce) me.push_back(meta_of(l, true));
-    for (int l : cn) mn.push_back(meta_of(l, false));
+    // faces in the order of tiles of 16 grid rows x 32 columns, row by row inside a tile: 128 of them
+    // are about 4 rows x 32, and their neighbours mostly each other
+    auto tiled = [&](std::vector<int> v) {
+      auto key = [&](int l) {
+        const int i = g->l2i[l - 1], j = g->l2j[l - 1];
+        return std::make_tuple(i / 16, j / 32, i, j);
+      };
+      std::stable_sort(v.begin(), v.end(), [&](int a, int b) { return key(a) < key(b); });
+      return v;
+    };
+    for (int l : tiled(ce)) me.push_back(meta_of(l, true));
+    for (int l : tiled(cn)) mn.push_back(meta_of(l, false));
+    rc |= build_tiles(c, me, &c->tce);
+    rc |= build_tiles(c, mn, &c->tcn);
     rc |= c->alloc(&c->mce, me.size());
     rc |= c->alloc(&c->mcn, mn.size());
     if (rc) { delete c; return rc; }
     if (!me.empty()) cudaMemcpy(c->mce, me.data(), me.size() * sizeof(FaceMeta), cudaMemcpyHostToDevice);
     if (!mn.empty()) cudaMemcpy(c->mcn, mn.data(), mn.size() * sizeof(FaceMeta), cudaMemcpyHostToDevice);
+    // Before the autotuner: the fused momentum kernel once its tiles give every SM one, else the split
+    // kernels, whose cells spread over all SMs (both directions of one call, split / fused: 31 tiles
+    // 75 / 81 us, 800 tiles 195 / 166 us, 1260 tiles 442 / 340 us)
+    if (c->tce.ntile < pr.multiProcessorCount) { c->tune.mom_cl = 8; c->tune.mom_nt = 64; }
   }
   rc = build_pcg(c, g);
   if (!rc) rc = c->alloc(&c->hist, (size_t)kHistSlots * (c->pcg.R.n + c->pcg.B.n + 2));
