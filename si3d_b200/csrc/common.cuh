@@ -36,6 +36,7 @@ struct Fields2 {
 struct Grid {
   int lm, lm1, km1, km, k1, P;
   const int *lEC, *lWC, *lNC, *lSC, *kmz;   // [P], 1-based neighbour columns, lm1 = dry
+  const int *kmu, *kmv;                     // [P], last layer of the east / north face, 0 where it is closed
   const double *hhs, *hhu, *hhv;            // [P]
   const double* zlevel;                     // [km1] (1-based via zl())
 };
@@ -120,13 +121,11 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_gr
 // Roe's superbee limiter (the reference always uses it, si3d_procedures.f90:2931-2934 in exsal,
 // :4186-4190 in exTracer); cf0 is the default C_f.
 __device__ __forceinline__ double superbee(double s1, double s2, double s3, double s4, double vel, double cf0) {
-  double C_f = cf0;
-  if (s3 - s2 != 0) {
-    const bool down = copysign(1.0, vel) > 0;  // gamma1 = -SIGN(1, vel)
-    const double ratio = down ? (s2 - s1) / (s3 - s2) : (s4 - s3) / (s3 - s2);
-    C_f = fmax(fmax(0., fmin(1., 2. * ratio)), fmin(2., ratio));
-  }
-  return C_f;
+  // (one division whatever the direction, and no branch: the lanes of a warp differ in both)
+  const bool down = copysign(1.0, vel) > 0;  // gamma1 = -SIGN(1, vel)
+  const double ratio = (down ? s2 - s1 : s4 - s3) / (s3 - s2);
+  const double C_f = fmax(fmax(0., fmin(1., 2. * ratio)), fmin(2., ratio));
+  return s3 - s2 != 0 ? C_f : cf0;
 }
 
 __device__ __forceinline__ double zmid(const Dev& d, int k, double hpk) {

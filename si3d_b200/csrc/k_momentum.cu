@@ -357,12 +357,10 @@ template <int NT>
 __global__ void __launch_bounds__(NT) k_mom_rho(Dev d) {
   const int l = blockIdx.x * NT + threadIdx.x + 1;
   if (l > d.g.lm) return;
-  const int lE = NB(d.g.lEC, l), lN = NB(d.g.lNC, l);
-  const int kz = NB(d.g.kmz, l), ku = d.s.k1u[l - 1], kv = d.s.k1v[l - 1];
-  const int kx = min(kz, NB(d.g.kmz, lE)), ky = min(kz, NB(d.g.kmz, lN));
+  const int ku = d.s.k1u[l - 1], kv = d.s.k1v[l - 1], kx = NB(d.g.kmu, l), ky = NB(d.g.kmv, l);
   double sx = 0, sy = 0;
 #pragma unroll 8
-  for (int k = min(ku, kv); k <= kz; ++k) {
+  for (int k = min(ku, kv); k <= max(kx, ky); ++k) {
     const double r = 1000 + d.f.rhop[IX(d, k, l)];
     if (k >= ku && k <= kx) sx += r;
     if (k >= kv && k <= ky) sy += r;
@@ -372,16 +370,15 @@ __global__ void __launch_bounds__(NT) k_mom_rho(Dev d) {
 }
 
 // Back substitution of the momentum systems, summing the depth totals on the way up (one thread per
-// face column).  A kernel of its own because it only streams: with no shared memory it keeps 64 warps
-// and the whole L1 for loads in flight, where the end of the fused kernel (16 warps, a ring that
-// leaves 28 KB of L1) took 0.36 ms a direction at 2000 x 1000 x 60 for five streams.
+// column).  A kernel of its own because it only streams: with no shared memory it keeps 64 warps and
+// the whole L1 for loads in flight, where the end of the fused kernel (16 warps, a ring that leaves
+// 28 KB of L1) took 0.36 ms a direction at 2000 x 1000 x 60 for five streams.
 template <int IEQ, int NT>
-__global__ void __launch_bounds__(NT) k_mom_back(Dev d, const FaceMeta* __restrict__ meta, int ncols) {
-  const int t = min((int)(blockIdx.x * NT + threadIdx.x), ncols - 1);
+__global__ void __launch_bounds__(NT) k_mom_back(Dev d) {
+  const int l0 = blockIdx.x * NT + threadIdx.x + 1, l = min(l0, d.g.lm);
   const bool X = (IEQ == 1);
-  const int l = __ldg(&meta[t].a.x), kmx = __ldg(&meta[t].b.z);
-  const int k1x = NB(X ? d.s.k1u : d.s.k1v, l);
-  const bool act = (int)(blockIdx.x * NT + threadIdx.x) < ncols && k1x <= kmx;
+  const int kmx = NB(X ? d.g.kmu : d.g.kmv, l), k1x = NB(X ? d.s.k1u : d.s.k1v, l);
+  const bool act = l0 <= d.g.lm && k1x <= kmx;
   double* __restrict__ agA = X ? d.f.agx : d.f.agy;
   double* __restrict__ arA = X ? d.f.arx : d.f.ary;
   const double* __restrict__ cc = d.scr;
@@ -720,7 +717,7 @@ void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const MomTiles& t
                 const ObcDev* obc, int nobc) {
   if (tu.mom_cl == 1 && nobc == 0) {   // one pass per column (open boundaries need the split kernels)
     k_mom_fused<IEQ><<<tiles.ntile, MT, kMomSmem, st>>>(d, cols, tiles);
-    k_mom_back<IEQ, BT><<<(ncols + BT - 1) / BT, BT, 0, st>>>(d, cols, ncols);
+    k_mom_back<IEQ, BT><<<(d.g.lm + BT - 1) / BT, BT, 0, st>>>(d);
     return;
   }
   const int g1 = (ncols + CW - 1) / CW;
@@ -736,7 +733,7 @@ void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const MomTiles& t
     case 256: k_mom_columns<IEQ, 256><<<(ncols + 255) / 256, 256, 0, st>>>(d, cols, ncols); break;
     default: k_mom_columns<IEQ, 128><<<(ncols + 127) / 128, 128, 0, st>>>(d, cols, ncols); break;
   }
-  k_mom_back<IEQ, BT><<<(ncols + BT - 1) / BT, BT, 0, st>>>(d, cols, ncols);
+  k_mom_back<IEQ, BT><<<(d.g.lm + BT - 1) / BT, BT, 0, st>>>(d);
 }
 
 void launch_momentum(const Dev& d, int ieq, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu,

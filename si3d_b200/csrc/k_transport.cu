@@ -5,8 +5,12 @@
 // :2181-2231), settrap (:3418-3618), settrap2 (:3944-4087), save (:3621-3941) with layer_hp2
 // (:2238-2292), TopLayerIndexp2 (:2368-2427), continuity(2) and densty_s.
 //
-// Every kernel gives one thread one water column and walks the layers; a warp covers 32
-// consecutive columns so each per-layer access of a layer-major field is coalesced.  Arrays that
+// A warp covers 32 consecutive columns and its lanes stay on one layer, so each per-layer access of a
+// layer-major field is coalesced; the sweeps that go up a column start at the deepest bottom among the
+// warp's columns, not each at its own.  Measured for that and for batches of loads, selects in place
+// of branches around the limiter, and no copies below the surface inside fd, at 2000 x 1000 x 60 per
+// call: scalar stage 1.48 -> 1.25 ms, velocity stage 0.68 -> 0.53, surface layer 0.34 -> 0.08,
+// continuity(2) 0.30 -> 0.18, zeta assembly 0.20 -> 0.16 ms.  Arrays that
 // the reference keeps across calls with partial rewrites (the thread-private flux arrays Bth2,
 // Bth3, Bth4, and uh/vh/h above the surface) are kept as persistent device fields and written
 // exactly where the reference writes them.
@@ -30,15 +34,16 @@ __device__ __forceinline__ bool nwet(const Dev& d, int l) { return NB(d.g.lNC, l
 // them 0 everywhere); its full-column loops rewrite those levels with identical values, so the
 // loops below stop at these limits and the state stays bit-identical.
 __device__ __forceinline__ int zlim(const Dev& d, int l) { return NB(d.g.kmz, l) + 1; }
-__device__ __forceinline__ int ulim(const Dev& d, int l) {
-  return ewet(d, l) ? min(NB(d.g.kmz, l), NB(d.g.kmz, NB(d.g.lEC, l))) : 0;
-}
-__device__ __forceinline__ int vlim(const Dev& d, int l) {
-  return nwet(d, l) ? min(NB(d.g.kmz, l), NB(d.g.kmz, NB(d.g.lNC, l))) : 0;
-}
+__device__ __forceinline__ int ulim(const Dev& d, int l) { return NB(d.g.kmu, l); }
+__device__ __forceinline__ int vlim(const Dev& d, int l) { return NB(d.g.kmv, l); }
 
 // ------------------------------------------------------------- slayer_h
-template <int CLN>
+// FULL: as the reference, every layer below the surface copied from hp, hup, hvp.  Inside fd those
+// copies only feed imsal (and the tracers, which ask for the full form) before vel2 writes every
+// layer k1 .. kmz again, so the short form leaves them out: it writes the surface layers, the layers
+// that vel2 does not reach (1 and kmz + 1) and h of layer k1z + 2, which imsal still reads from h
+// (it takes deeper layers from hp).  At 2000 x 1000 x 60: 334 us for six streams, FULL.
+template <int CLN, bool FULL>
 __global__ void __launch_bounds__(32 * CLN) k_slayer_h(Dev d) {
   double* __restrict__ f_h = d.f.h;
   double* __restrict__ f_hp = d.f.hp;
@@ -54,6 +59,7 @@ __global__ void __launch_bounds__(32 * CLN) k_slayer_h(Dev d) {
   double* __restrict__ h = f_h; double* __restrict__ hu = f_hu; double* __restrict__ hv = f_hv;
   const double* __restrict__ hp = f_hp; const double* __restrict__ hup = f_hup; const double* __restrict__ hvp = f_hvp;
   const int zL = zlim(d, l), uL = ulim(d, l), vL = vlim(d, l);
+  if (FULL) {
   #pragma unroll 4
   for (int k = 1 + ty; k <= min(kz - 1, zL); k += CLN) h[IX(d, k, l)] = hp[IX(d, k, l)];
   #pragma unroll 4
@@ -66,6 +72,13 @@ __global__ void __launch_bounds__(32 * CLN) k_slayer_h(Dev d) {
   for (int k = ku + 1 + ty; k <= uL; k += CLN) hu[IX(d, k, l)] = hup[IX(d, k, l)];
   #pragma unroll 4
   for (int k = kv + 2 + ty; k <= vL; k += CLN) hv[IX(d, k, l)] = hvp[IX(d, k, l)];
+  } else {
+    if (1 <= min(kz - 1, zL)) h[IX(d, 1, l)] = hp[IX(d, 1, l)];
+    if (1 <= min(ku - 1, uL)) hu[IX(d, 1, l)] = hup[IX(d, 1, l)];
+    if (1 <= min(kv - 1, vL)) hv[IX(d, 1, l)] = hvp[IX(d, 1, l)];
+    if (kz + 2 < zL) h[IX(d, kz + 2, l)] = hp[IX(d, kz + 2, l)];
+    if (kz + 2 <= zL || kz - 1 >= zL) h[IX(d, zL, l)] = hp[IX(d, zL, l)];
+  }
   // the copies above leave out the surface layers written below, so the lanes never overlap
   if (ty != 0) return;
   // Surface layers.  A column whose surface index has reached the bottom level (every layer
@@ -109,41 +122,44 @@ __global__ void __launch_bounds__(32 * CLN) k_slayer_h(Dev d) {
 }
 
 // ------------------------------------------------------------- vel (uh, vh, k1u, k1v)
-template <int IEQ, int CLN>
-__global__ void __launch_bounds__(32 * CLN) k_vel_uv(Dev d, const int* __restrict__ cols, int ncols) {
-  double* __restrict__ f_agx = d.f.agx;
-  double* __restrict__ f_agy = d.f.agy;
-  double* __restrict__ f_arx = d.f.arx;
-  double* __restrict__ f_ary = d.f.ary;
-  double* __restrict__ f_hu = d.f.hu;
-  double* __restrict__ f_hv = d.f.hv;
-  double* __restrict__ f_uh = d.f.uh;
-  double* __restrict__ f_vh = d.f.vh;
-  const int t = blockIdx.x * 32 + threadIdx.x, ty = threadIdx.y;
-  const bool act = t < ncols;
-  const bool X = IEQ == 1;
-  int l = 0, k0 = 0;
-  int* k1 = X ? d.s.k1u : d.s.k1v;
-  double* uv = X ? f_uh : f_vh;
-  if (act) {
-    l = cols[t];
-    const int lO = X ? NB(d.g.lEC, l) : NB(d.g.lNC, l);
-    const int kmx = min(NB(d.g.kmz, lO), NB(d.g.kmz, l));
-    k0 = k1[l - 1];
-    const double gth = (X ? d.p.gdtdx : d.p.gdtdy) * d.tz;
-    const double c = gth * 1000. * (d.s.s[lO - 1] - d.s.s[l - 1]);
-    const double* ag = X ? f_agx : f_agy;
-    const double* ar = X ? f_arx : f_ary;
-#pragma unroll 4
-    for (int k = k0 + ty; k <= kmx; k += CLN) uv[IX(d, k, l)] = ag[IX(d, k, l)] - c * ar[IX(d, k, l)];
+// One thread per column, U layers in flight.
+template <int IEQ>
+__global__ void __launch_bounds__(TB) k_vel_uv(Dev d) {
+  const int l = blockIdx.x * TB + threadIdx.x + 1;
+  if (l > d.g.lm) return;
+  constexpr bool X = IEQ == 1;
+  const int kmx = X ? ulim(d, l) : vlim(d, l), lO = X ? NB(d.g.lEC, l) : NB(d.g.lNC, l);
+  if (kmx == 0) return;   // a closed face
+  int* __restrict__ k1 = X ? d.s.k1u : d.s.k1v;
+  double* __restrict__ uv = X ? d.f.uh : d.f.vh;
+  const double* __restrict__ huv = X ? d.f.hu : d.f.hv;
+  const double* __restrict__ ag = X ? d.f.agx : d.f.agy;
+  const double* __restrict__ ar = X ? d.f.arx : d.f.ary;
+  const int k0 = k1[l - 1];
+  const double gth = (X ? d.p.gdtdx : d.p.gdtdy) * d.tz;
+  const double c = gth * 1000. * (d.s.s[lO - 1] - d.s.s[l - 1]);
+  constexpr int U = 8;   // layers in flight
+  double top = 0.0, next = 0.0;   // the values of layers k0 and k0 + 1
+  for (int k = k0; k <= kmx; k += U) {
+    double g[U], r[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u <= kmx) { g[u] = ag[IX(d, k + u, l)]; r[u] = ar[IX(d, k + u, l)]; }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (k + u > kmx) break;
+      const double v = g[u] - c * r[u];
+      uv[IX(d, k + u, l)] = v;
+      if (k + u == k0) top = v;
+      if (k + u == k0 + 1) next = v;
+    }
   }
-  __syncthreads();   // the surface correction reads layers written by other lanes
-  if (!act || ty != 0) return;
-  const double* huv = X ? f_hu : f_hv;
-  // (a face column with every layer dry, k0 = km1, is never reached: the reference would write
-  //  past the last level there)
+  // the surface layer has dried: its transport goes to the layer below (a face column with every layer
+  // dry, k0 = km1, is never reached: the reference would write past the last level there)
   if (k0 < d.g.km1 && huv[IX(d, k0, l)] <= ZERO) {
-    uv[IX(d, k0 + 1, l)] = uv[IX(d, k0, l)] + uv[IX(d, k0 + 1, l)];
+    if (k0 > kmx) top = uv[IX(d, k0, l)];
+    if (k0 + 1 > kmx) next = uv[IX(d, k0 + 1, l)];
+    uv[IX(d, k0 + 1, l)] = top + next;
     uv[IX(d, k0, l)] = 0.0;
     k1[l - 1] = k0 + 1;
   }
@@ -196,18 +212,79 @@ __global__ void __launch_bounds__(32 * CLN) k_cont(Dev d) {
     }
   }
   __syncthreads();
-  if (ty != 0 || !act) return;
-  if (wet) {
+  // the sums, over every column of the warp from its deepest layer up, in place of the x terms
+  const int kw = __reduce_max_sync(0xffffffffu, wet ? kms : 0);
+  if (ty == 0) {
     double w = 0.0;
+    if (wet) {
 #pragma unroll 4
-    for (int k = kms; k > k1s; --k) {
-      w = w - s_x[k * 32 + cx] - s_y[k * 32 + cx];
-      wp[IX(d, k, l)] = w;
+      for (int k = kms; k > k1s; --k) {
+        w = w - s_x[k * 32 + cx] - s_y[k * 32 + cx];
+        s_x[k * 32 + cx] = w;
+      }
+      // level k1s: its own term, then the dry levels above it folded in (the reference stores the
+      // first sum and overwrites it with the second)
+      double ws = w - s_x[k1s * 32 + cx] - s_y[k1s * 32 + cx];
+      for (int k = d.g.k1; k <= k1s - 1; ++k) ws = ws - s_x[k * 32 + cx] - s_y[k * 32 + cx];
+      s_x[k1s * 32 + cx] = ws;
     }
-    // level k1s: its own term, then the dry levels above it folded in (the reference stores the
-    // first sum and overwrites it with the second)
-    double ws = w - s_x[k1s * 32 + cx] - s_y[k1s * 32 + cx];
-    for (int k = d.g.k1; k <= k1s - 1; ++k) ws = ws - s_x[k * 32 + cx] - s_y[k * 32 + cx];
+  }
+  __syncthreads();
+  // (a store of a layer is one run; stored by the summing lanes, each at its own depth, it was up to 32)
+  for (int k = kw - ty; k >= d.g.k1; k -= CLN)
+    if (wet && k >= k1s && k <= kms) wp[IX(d, k, l)] = s_x[k * 32 + cx];
+  if (CONT1 && act && ty == 0 && d.f.h[IX(d, k1s, l)] <= ZERO) d.s.k1z[l - 1] = min(k1s + 1, d.g.km1);
+}
+
+// The same with one thread per column, U layers' fluxes in flight and no shared memory, the lanes of a
+// warp going up together from the deepest of their columns (same operations in the same order).
+template <bool CONT1>
+__global__ void __launch_bounds__(TB) k_cont_column(Dev d) {
+  const int l0 = blockIdx.x * TB + threadIdx.x + 1, l = min(l0, d.g.lm);
+  const bool act = l0 <= d.g.lm;
+  const int kms = NB(d.g.kmz, l), k1s = d.s.k1z[l - 1], P = d.g.P, k1 = d.g.k1;
+  const bool wet = act && k1s <= kms;
+  const int dW = NB(d.g.lWC, l) - l, dS = NB(d.g.lSC, l) - l;
+  double* __restrict__ wp = d.f.wp;
+  const double* __restrict__ fx = CONT1 ? d.f.uh : d.f.uhp;
+  const double* __restrict__ fy = CONT1 ? d.f.vh : d.f.vhp;
+  const double* __restrict__ fx2 = d.f.uhpp;
+  const double* __restrict__ fy2 = d.f.vhpp;
+  if (wet)
+    for (int k = 1; k < k1s; ++k) wp[IX(d, k, l)] = 0.0;   // wp below kms is never non-zero
+  const int kw = __reduce_max_sync(0xffffffffu, wet ? kms : 0);
+  constexpr int U = CONT1 ? 2 : 4;   // layers in flight
+  double w = 0.0, ws = 0.0;
+  // down to level k1s each level's sum is stored; the dry levels above are folded into level k1s
+  for (int kb = kw; kb >= k1; kb -= U) {
+    double a0[U], a1[U], a2[U], a3[U], b0[U], b1[U], b2[U], b3[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = kb - u, ik = IX(d, k, l);
+      if (!wet || k > kms || k < k1) continue;
+      a0[u] = fx[ik]; a1[u] = fx[ik + dW];
+      b0[u] = fy[ik]; b1[u] = fy[ik + dS];
+      if (CONT1) { a2[u] = fx2[ik]; a3[u] = fx2[ik + dW]; b2[u] = fy2[ik]; b3[u] = fy2[ik + dS]; }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = kb - u;
+      if (!wet || k > kms || k < k1s) continue;
+      const double tx = CONT1 ? (a0[u] - a1[u] + a2[u] - a3[u]) / d.p.twodx : (a0[u] - a1[u]) / d.p.dx;
+      const double ty = CONT1 ? (b0[u] - b1[u] + b2[u] - b3[u]) / d.p.twody : (b0[u] - b1[u]) / d.p.dy;
+      w = w - tx - ty;
+      if (k > k1s) wp[IX(d, k, l)] = w;
+      else ws = w;
+    }
+  }
+  if (!act) return;
+  if (wet) {
+    for (int k = k1; k <= k1s - 1; ++k) {
+      const int ik = IX(d, k, l);
+      const double tx = CONT1 ? (fx[ik] - fx[ik + dW] + fx2[ik] - fx2[ik + dW]) / d.p.twodx : (fx[ik] - fx[ik + dW]) / d.p.dx;
+      const double ty = CONT1 ? (fy[ik] - fy[ik + dS] + fy2[ik] - fy2[ik + dS]) / d.p.twody : (fy[ik] - fy[ik + dS]) / d.p.dy;
+      ws = ws - tx - ty;
+    }
     wp[IX(d, k1s, l)] = ws;
   }
   if (CONT1 && d.f.h[IX(d, k1s, l)] <= ZERO) d.s.k1z[l - 1] = min(k1s + 1, d.g.km1);
@@ -259,35 +336,36 @@ __global__ void __launch_bounds__(32 * CLN) k_exsal_flux(Dev d, const double* __
     const double sU = sp[ik - P], sUU = sp[ik2], sD = sp[ik + P];
     const double hW = hpp[ik + dW], hEE = hpp[ik + dEE], hS = hpp[ik + dS], hNN = hpp[ik + dNN];
     const double hUU = hpp[ik2], hD = hpp[ik + P];
-    // EW
-    if (hu > ZERO) {
+    // (each face's flux formed whether or not the face is wet, and dropped where it is dry: the lanes
+    // of a warp differ, and what is dropped may be infinite)
+    {   // EW
       const double vel = (uo + un) / 2.;
       const double s3 = sE;
       const double s1 = (hW <= ZERO) ? s2 : sW;
       const double s4 = (hEE <= ZERO) ? s3 : sEE;
       const double C_f = superbee(s1, s2, s3, s4, vel, 0.0);
-      B2[ik] = vel / 2. * (s3 + s2) - ((1. - C_f) * fabs(vel) + vel * vel * twodt1 * d.p.rdx * C_f) * (s3 - s2) / 2.;
-    } else B2[ik] = 0.0;
-    // NS
-    if (hv > ZERO) {
+      const double f = vel / 2. * (s3 + s2) - ((1. - C_f) * fabs(vel) + vel * vel * twodt1 * d.p.rdx * C_f) * (s3 - s2) / 2.;
+      B2[ik] = hu > ZERO ? f : 0.0;
+    }
+    {   // NS
       const double vel = (vo + vn) / 2.;
       const double s3 = sN;
       const double s1 = (hS <= ZERO) ? s2 : sS;
       const double s4 = (hNN <= ZERO) ? s3 : sNN;
       const double C_f = superbee(s1, s2, s3, s4, vel, 0.0);
-      B4[ik] = vel / 2. * (s3 + s2) - ((1. - C_f) * fabs(vel) + vel * vel * twodt1 * d.p.rdy * C_f) * (s3 - s2) / 2.;
-    } else B4[ik] = 0.0;
-    // UD (hp(1, l) is never positive, so k-2 >= 1 whenever this branch is taken)
-    if (hpu > ZERO) {
-      double vel = wk;
-      if (k == k1s) vel = 0.0;
+      const double f = vel / 2. * (s3 + s2) - ((1. - C_f) * fabs(vel) + vel * vel * twodt1 * d.p.rdy * C_f) * (s3 - s2) / 2.;
+      B4[ik] = hv > ZERO ? f : 0.0;
+    }
+    {   // UD (hp(1, l) is never positive, so k-2 >= 1 whenever this flux is kept)
+      const double vel = k == k1s ? 0.0 : wk;
       const double s3 = sU;
       const double s4 = (k - 2 < 1 || hUU <= ZERO) ? s3 : sUU;
       const double s1 = (hD <= ZERO) ? s2 : sD;
       const double C_f = superbee(s1, s2, s3, s4, vel, 1.0);
       const double delz = (hpk + hpu) / 2.;
-      B3[ik] = vel / 2. * (s3 + s2) - ((1. - C_f) * fabs(vel) + vel * vel * twodt1 / delz * C_f) * (s3 - s2) / 2.;
-    } else B3[ik] = 0.0;
+      const double f = vel / 2. * (s3 + s2) - ((1. - C_f) * fabs(vel) + vel * vel * twodt1 / delz * C_f) * (s3 - s2) / 2.;
+      B3[ik] = hpu > ZERO ? f : 0.0;
+    }
   }
 }
 
@@ -341,16 +419,15 @@ __global__ void __launch_bounds__(32 * CLN) k_exsal_rhs(Dev d) {
   }
 }
 
-// imsal's vertical-diffusion tridiagonal solve per column (trid1), right-hand side read from sal.
+// imsal's vertical-diffusion tridiagonal solve per column (trid1), right-hand side read from sal.  hd:
+// the field that holds h from layer k1z + 2 down (h itself, or hp inside fd, see k_slayer_h).
 template <int NTB>
-__global__ void __launch_bounds__(NTB) k_imsal(Dev d) {
+__global__ void __launch_bounds__(NTB) k_imsal(Dev d, const double* __restrict__ hd) {
   constexpr int RD = 4;                // layers in flight in the forward sweep
   __shared__ double ring[RD][3][NTB];  // [slot][input][thread]: a thread's slots are its own
-  const int l = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (l > d.g.lm) return;
+  const int l0 = blockIdx.x * blockDim.x + threadIdx.x + 1, l = min(l0, d.g.lm);
   const int kms = NB(d.g.kmz, l), k1s = d.s.k1z[l - 1];
-  const int nw = kms - k1s + 1;
-  if (nw < 1) return;
+  const int nw = l0 > d.g.lm ? 0 : kms - k1s + 1;
   const int P = d.g.P;
   const double twodt1 = d.p.twodt * d.tz;
   const double* __restrict__ sp = d.f.salpp;
@@ -358,82 +435,87 @@ __global__ void __launch_bounds__(NTB) k_imsal(Dev d) {
   const double* __restrict__ Dv = d.f.Dv;
   double* __restrict__ sal = d.f.sal;
   double* __restrict__ esc = d.scr;
-  // layer thickness at time n with the surface corrections (:3128-3132)
-  const double hpp_k1 = d.f.hpp[IX(d, k1s, l)];
-  auto hn = [&](int k) -> double {
-    if (k == k1s) return twodt1 * d.f.wp[IX(d, k1s, l)] + hpp_k1;
-    if (k == k1s + 1 && hpp_k1 <= ZERO) return d.f.hpp[IX(d, k1s + 1, l)];
-    return h[IX(d, k, l)];
-  };
   if (nw == 1) {
-    const double a2 = hn(k1s) / twodt1;
+    // thickness at time n with the surface corrections (:3128-3132)
+    const double a2 = (twodt1 * d.f.wp[IX(d, k1s, l)] + d.f.hpp[IX(d, k1s, l)]) / twodt1;
     const double ds = sal[IX(d, k1s, l)];
     double v = ds / a2;
     if (h[IX(d, k1s, l)] < 1.E-2) v = sp[IX(d, k1s, l)];
     sal[IX(d, k1s, l)] = v;
-    return;
   }
-  // trid1 forward sweep: e in scratch, f in sal.  Iteration k reads sal(k), Dv(k + 1) and h(k + 1);
-  // these are copied into this thread's slots of a shared-memory ring by cp.async, RD layers ahead.
-  // 1 / (hn(k) + hn(k+1)) is shared with the next layer's a1, so a layer takes two divisions.
-  const double rt = 1.0 / twodt1;
-  const int tid = threadIdx.x;
-  auto issue = [&](int kk, int slot) {
-    const int ikk = IX(d, kk, l);
-    cp_async8(&ring[slot][0][tid], &sal[ikk]);
-    cp_async8(&ring[slot][1][tid], &Dv[ikk + P]);
-    cp_async8(&ring[slot][2][tid], &h[ikk + P]);
-  };
+  const bool act = nw >= 2;
+  double x = 0.0;   // the bottom layer's solution
+  if (act) {
+    const double hpp_k1 = d.f.hpp[IX(d, k1s, l)];
+    // trid1 forward sweep: e in scratch, f in sal.  Iteration k reads sal(k), Dv(k + 1) and h(k + 1);
+    // these are copied into this thread's slots of a shared-memory ring by cp.async, RD layers ahead.
+    // 1 / (hn(k) + hn(k+1)) is shared with the next layer's a1, so a layer takes two divisions.
+    const double rt = 1.0 / twodt1;
+    const int tid = threadIdx.x;
+    auto issue = [&](int kk, int slot) {
+      const int ikk = IX(d, kk, l);
+      cp_async8(&ring[slot][0][tid], &sal[ikk]);
+      cp_async8(&ring[slot][1][tid], &Dv[ikk + P]);
+      if (kk > k1s) cp_async8(&ring[slot][2][tid], &hd[ikk + P]);   // layer k1s + 2 on
+    };
 #pragma unroll
-  for (int j = 0; j < RD; ++j) {   // one commit group per layer (empty past the bottom)
-    if (k1s + j <= kms) issue(k1s + j, j);
-    cp_async_commit();
-  }
-  const double hn1 = hn(k1s + 1);  // the second layer's thickness carries the surface correction
-  double hn_k = hn(k1s), e_prev = 0, f_prev = 0, rkm = 0.0, dvk = Dv[IX(d, k1s, l)];
-  int ik = IX(d, k1s, l);
-  for (int k = k1s, slot = 0; k <= kms; ++k, ik += P, slot = (slot + 1 == RD) ? 0 : slot + 1) {
-    cp_async_wait<RD - 1>();     // layer k's group has landed (this thread's own copies)
-    const double ds = ring[slot][0][tid], dvkp = ring[slot][1][tid];
-    const double hn_kp = (k < kms) ? ((k == k1s) ? hn1 : ring[slot][2][tid]) : 0.0;
-    const double rkp = (k < kms) ? 1.0 / (hn_k + hn_kp) : 0.0;
-    const double a3 = (k < kms) ? -dvkp * rkp * 2. : 0.0;
-    double a1 = 0.0;
-    if (k > k1s) a1 = -dvk * rkm * 2.;
-    const double a2 = hn_k * rt - a1 - a3;
-    const int kk = k - k1s + 1;
-    if (kk == 1) {
-      const double r = 1.0 / a2;
-      e_prev = -a3 * r;
-      f_prev = ds * r;
-      esc[ik] = e_prev;
-      sal[ik] = f_prev;
-    } else {
-      const double r = 1.0 / (a2 + a1 * e_prev);
-      const double f = (ds - a1 * f_prev) * r;
-      sal[ik] = f;
-      if (kk < nw) {
-        const double e = -a3 * r;
-        esc[ik] = e;
-        e_prev = e; f_prev = f;
-      }
+    for (int j = 0; j < RD; ++j) {   // one commit group per layer (empty past the bottom)
+      if (k1s + j <= kms) issue(k1s + j, j);
+      cp_async_commit();
     }
-    // refill the slot with layer k + RD (its values are consumed: the stores above depend on them)
-    if (k + RD <= kms) issue(k + RD, slot);
-    cp_async_commit();
-    hn_k = hn_kp;
-    rkm = rkp;
-    dvk = dvkp;
+    // the first two layers' thicknesses carry the surface corrections (:3128-3132)
+    const double hn1 = (hpp_k1 <= ZERO) ? d.f.hpp[IX(d, k1s + 1, l)] : h[IX(d, k1s + 1, l)];
+    double hn_k = twodt1 * d.f.wp[IX(d, k1s, l)] + hpp_k1;
+    double e_prev = 0, rkm = 0.0, dvk = Dv[IX(d, k1s, l)];
+    int ik = IX(d, k1s, l);
+    for (int k = k1s, slot = 0; k <= kms; ++k, ik += P, slot = (slot + 1 == RD) ? 0 : slot + 1) {
+      cp_async_wait<RD - 1>();     // layer k's group has landed (this thread's own copies)
+      const double ds = ring[slot][0][tid], dvkp = ring[slot][1][tid];
+      const double hn_kp = (k < kms) ? ((k == k1s) ? hn1 : ring[slot][2][tid]) : 0.0;
+      const double rkp = (k < kms) ? 1.0 / (hn_k + hn_kp) : 0.0;
+      const double a3 = (k < kms) ? -dvkp * rkp * 2. : 0.0;
+      double a1 = 0.0;
+      if (k > k1s) a1 = -dvk * rkm * 2.;
+      const double a2 = hn_k * rt - a1 - a3;
+      const double r = 1.0 / (a2 + a1 * e_prev);
+      x = (k == k1s) ? ds * r : (ds - a1 * x) * r;
+      sal[ik] = x;
+      if (k < kms) {
+        e_prev = -a3 * r;
+        esc[ik] = e_prev;
+      }
+      // refill the slot with layer k + RD (its values are consumed: the stores above depend on them)
+      if (k + RD <= kms) issue(k + RD, slot);
+      cp_async_commit();
+      hn_k = hn_kp;
+      rkm = rkp;
+      dvk = dvkp;
+    }
+    cp_async_wait<0>();
   }
-  double nxt = sal[IX(d, kms, l)];
-#pragma unroll 4
-  for (int k = kms - 1; k >= k1s; --k) {
-    nxt = esc[IX(d, k, l)] * nxt + sal[IX(d, k, l)];
-    sal[IX(d, k, l)] = nxt;
+  // back substitution: the lanes of a warp go up together from the deepest of their columns, so that
+  // a load or store of a layer is one run (each lane from its own bottom: up to 32 layers at once)
+  const double bottom = x;
+  const int kw = __reduce_max_sync(0xffffffffu, act ? kms : 0), kt = __reduce_min_sync(0xffffffffu, act ? k1s : 1 << 20);
+  constexpr int U = 4;   // layers in flight
+  for (int k0 = kw - 1; k0 >= kt; k0 -= U) {
+    double e[U], f[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 - u, ik = IX(d, k, l);
+      if (act && k >= k1s && k < kms) { e[u] = esc[ik]; f[u] = sal[ik]; }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const int k = k0 - u;
+      if (!act || k < k1s || k >= kms) continue;
+      x = e[u] * x + f[u];
+      sal[IX(d, k, l)] = x;
+    }
   }
-  const double top = sal[IX(d, k1s, l)];
-  for (int k = d.g.k1; k <= k1s - 1; ++k) sal[IX(d, k, l)] = top;
-  sal[IX(d, kms + 1, l)] = sal[IX(d, kms, l)];
+  if (!act) return;
+  for (int k = d.g.k1; k <= k1s - 1; ++k) sal[IX(d, k, l)] = x;
+  sal[IX(d, kms + 1, l)] = bottom;
 }
 
 // ------------------------------------------------------------- vel2 (layer_h + wetting)
@@ -447,35 +529,19 @@ __global__ void __launch_bounds__(32 * CLN) k_vel2(Dev d) {
   const int l = blockIdx.x * 32 + threadIdx.x + 1, ty = threadIdx.y;
   const bool act = l <= d.g.lm;
   if (act) {
-    const int kms = NB(d.g.kmz, l);
+    const int kms = NB(d.g.kmz, l), kmx = ulim(d, l), kmy = vlim(d, l);   // 0 at closed faces
     const double sl = d.s.s[l - 1];
+    const double hhs = d.g.hhs[l - 1], hhu = d.g.hhu[l - 1], hhv = d.g.hhv[l - 1];
+    const double sx = fmax(sl, d.s.s[NB(d.g.lEC, l) - 1]), sy = fmax(sl, d.s.s[NB(d.g.lNC, l) - 1]);
 #pragma unroll 4
-    for (int k = d.g.k1 + ty; k <= kms; k += CLN) {
-      double v = fmin(zl(d, k + 1), d.g.hhs[l - 1]) - fmax(zl(d, k), -sl);
-      if (v <= HMIN) v = ZERO;
-      f_h[IX(d, k, l)] = v;
-    }
-    if (ewet(d, l)) {
-      const int lE = NB(d.g.lEC, l);
-      const int kmx = min(kms, NB(d.g.kmz, lE));
-      const double sm = fmax(sl, d.s.s[lE - 1]);
-  #pragma unroll 4
-      for (int k = d.g.k1 + ty; k <= kmx; k += CLN) {
-        double v = fmin(zl(d, k + 1), d.g.hhu[l - 1]) - fmax(zl(d, k), -sm);
-        if (v <= HMIN) v = ZERO;
-        f_hu[IX(d, k, l)] = v;
-      }
-    }
-    if (nwet(d, l)) {
-      const int lN = NB(d.g.lNC, l);
-      const int kmy = min(kms, NB(d.g.kmz, lN));
-      const double sm = fmax(sl, d.s.s[lN - 1]);
-  #pragma unroll 4
-      for (int k = d.g.k1 + ty; k <= kmy; k += CLN) {
-        double v = fmin(zl(d, k + 1), d.g.hhv[l - 1]) - fmax(zl(d, k), -sm);
-        if (v <= HMIN) v = ZERO;
-        f_hv[IX(d, k, l)] = v;
-      }
+    for (int k = d.g.k1 + ty; k <= kms; k += CLN) {   // the three thicknesses of a layer share its bounds
+      const int ik = IX(d, k, l);
+      const double zt = zl(d, k), zb = zl(d, k + 1);
+      const double v = fmin(zb, hhs) - fmax(zt, -sl);
+      const double wu = fmin(zb, hhu) - fmax(zt, -sx), wv = fmin(zb, hhv) - fmax(zt, -sy);
+      f_h[ik] = v <= HMIN ? ZERO : v;
+      if (k <= kmx) f_hu[ik] = wu <= HMIN ? ZERO : wu;
+      if (k <= kmy) f_hv[ik] = wv <= HMIN ? ZERO : wv;
     }
   }
   __syncthreads();   // the surface corrections read layers written by other lanes
@@ -830,12 +896,20 @@ static inline int grid_of(int n) { return (n + TB - 1) / TB; }
 constexpr int BK_LANES = 4;   // layer lanes of the copy kernels (slayer_h, vel_uv, vel2)
 constexpr int HALF_LANES = 2;   // layer lanes of k_half_level and k_save
 constexpr int CONT_LANES = 8;   // layer lanes of the continuity kernels (4 and 16 measured slower)
+// From this many columns on one thread per column fills the chip and the lanes' shared-memory planes only
+// take L1 from the loads in flight (velocity stage / continuity(2): 1.4e6 columns 629 / 304 -> 562 / 180 us,
+// 350000 144 / 50 -> 130 / 28 us, 102417 46 / 14 -> 44 / 12 us; 3924 columns 25 -> 31 us the other way).
+constexpr int CONT_COLUMN = 65536;
 
 // Shared memory of a continuity block: two planes of km1 + 1 levels x 32 columns.
 static size_t cont_smem(int km1) { return 2 * (size_t)(km1 + 1) * 32 * sizeof(double); }
 
 template <bool CONT1>
 static void launch_cont(const Dev& d, cudaStream_t st) {
+  if (d.g.lm >= CONT_COLUMN) {
+    k_cont_column<CONT1><<<grid_of(d.g.lm), TB, 0, st>>>(d);
+    return;
+  }
   k_cont<CONT_LANES, CONT1><<<(d.g.lm + 31) / 32, dim3(32, CONT_LANES), cont_smem(d.g.km1), st>>>(d);
 }
 
@@ -851,28 +925,30 @@ int transport_init(int km1) {
   return 0;
 }
 
-void launch_slayer_h(const Dev& d, cudaStream_t st) {
-  k_slayer_h<BK_LANES><<<(d.g.lm + 31) / 32, dim3(32, BK_LANES), 0, st>>>(d);
+void launch_slayer_h(const Dev& d, bool full, cudaStream_t st) {
+  if (full) k_slayer_h<BK_LANES, true><<<(d.g.lm + 31) / 32, dim3(32, BK_LANES), 0, st>>>(d);
+  else k_slayer_h<1, false><<<(d.g.lm + 31) / 32, dim3(32, 1), 0, st>>>(d);
 }
 
-void launch_vel(const Dev& d, const int* ce, int nce, const int* cn, int ncn, cudaStream_t st) {
-  if (nce > 0) k_vel_uv<1, BK_LANES><<<(nce + 31) / 32, dim3(32, BK_LANES), 0, st>>>(d, ce, nce);
-  if (ncn > 0) k_vel_uv<2, BK_LANES><<<(ncn + 31) / 32, dim3(32, BK_LANES), 0, st>>>(d, cn, ncn);
+void launch_vel(const Dev& d, cudaStream_t st) {
+  k_vel_uv<1><<<grid_of(d.g.lm), TB, 0, st>>>(d);
+  k_vel_uv<2><<<grid_of(d.g.lm), TB, 0, st>>>(d);
   launch_cont<true>(d, st);
 }
 
-void launch_exsal_imsal(const Dev& d, const Tune& tu, cudaStream_t st) {
+void launch_exsal_imsal(const Dev& d, const Tune& tu, bool h_from_hp, cudaStream_t st) {
   const int cg = (d.g.lm + 31) / 32;
   const double* sp = d.f.salpp;
+  const double* hd = h_from_hp ? d.f.hp : d.f.h;
   switch (tu.sal_cl) {
     case 2: k_exsal_flux<2><<<cg, dim3(32, 2), 0, st>>>(d, sp); k_exsal_rhs<2><<<cg, dim3(32, 2), 0, st>>>(d); break;
     case 4: k_exsal_flux<4><<<cg, dim3(32, 4), 0, st>>>(d, sp); k_exsal_rhs<4><<<cg, dim3(32, 4), 0, st>>>(d); break;
     default: k_exsal_flux<8><<<cg, dim3(32, 8), 0, st>>>(d, sp); k_exsal_rhs<8><<<cg, dim3(32, 8), 0, st>>>(d); break;
   }
   switch (tu.sal_nt) {
-    case 64: k_imsal<64><<<(d.g.lm + 63) / 64, 64, 0, st>>>(d); break;
-    case 256: k_imsal<256><<<(d.g.lm + 255) / 256, 256, 0, st>>>(d); break;
-    default: k_imsal<128><<<(d.g.lm + 127) / 128, 128, 0, st>>>(d); break;
+    case 64: k_imsal<64><<<(d.g.lm + 63) / 64, 64, 0, st>>>(d, hd); break;
+    case 256: k_imsal<256><<<(d.g.lm + 255) / 256, 256, 0, st>>>(d, hd); break;
+    default: k_imsal<128><<<(d.g.lm + 127) / 128, 128, 0, st>>>(d, hd); break;
   }
 }
 

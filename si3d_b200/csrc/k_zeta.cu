@@ -30,8 +30,8 @@ namespace si3d {
 
 // ------------------------------------------------------------------ matcon
 __global__ void k_matcon(Dev d) {
-  double* __restrict__ f_uhpp = d.f.uhpp;
-  double* __restrict__ f_vhpp = d.f.vhpp;
+  const double* __restrict__ f_uhpp = d.f.uhpp;
+  const double* __restrict__ f_vhpp = d.f.vhpp;
   const int l = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (l > d.g.lm) return;
   const double tz = d.tz;
@@ -56,10 +56,19 @@ __global__ void k_matcon(Dev d) {
   const int kms = NB(d.g.kmz, l);
   const double rdx = 1.0 / d.p.dx, rdy = 1.0 / d.p.dy;   // divisions by the grid constants as products
   double sum = 0;
-  #pragma unroll 4
-  for (int k = d.g.k1; k <= kms; ++k)
-    sum += (f_uhpp[IX(d, k, l)] - f_uhpp[IX(d, k, lW)]) * rdx +
-           (f_vhpp[IX(d, k, l)] - f_vhpp[IX(d, k, lS)]) * rdy;
+  constexpr int U = 8;   // layers in flight (a batch of four waited twice as often for memory)
+  for (int k = d.g.k1; k <= kms; k += U) {
+    double u0[U], u1[U], v0[U], v1[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u <= kms) {
+        u0[u] = f_uhpp[IX(d, k + u, l)]; u1[u] = f_uhpp[IX(d, k + u, lW)];
+        v0[u] = f_vhpp[IX(d, k + u, l)]; v1[u] = f_vhpp[IX(d, k + u, lS)];
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u <= kms) sum += (u0[u] - u1[u]) * rdx + (v0[u] - v1[u]) * rdy;
+  }
   const double ddv = dt1 * sum;
   d.s.dd[l - 1] = ddv;
   d.s.qq[l - 1] = d.s.spp[l - 1] - dtdx1 * (d.s.eagx[l - 1] - d.s.eagx[lW - 1]) -
@@ -68,7 +77,7 @@ __global__ void k_matcon(Dev d) {
 }
 
 void launch_matcon(const Dev& d, cudaStream_t st) {
-  const int B = 256;
+  const int B = 128;
   k_matcon<<<(d.g.lm + B - 1) / B, B, 0, st>>>(d);
 }
 

@@ -52,7 +52,7 @@ using PcgDevF = PcgDevT<float>;
 // them): layer lanes per column of the cell-parallel kernels (2, 4, 8; momentum 1: the fused kernel)
 // and threads per block of the column-sequential kernels (64, 128, 256).
 struct Tune {
-  int mom_cl = 1, mom_nt = 128, sal_cl = 8, sal_nt = 128;
+  int mom_cl = 1, mom_nt = 128, sal_cl = 4, sal_nt = 64;
 };
 
 // Static indices of one u (v) face column of the momentum stage, computed once from the grid maps
@@ -181,9 +181,11 @@ int pcg_loop(const PcgDev& P, GridBar* bar, int nblocks, bool test2, cudaStream_
              const GridBar* init = nullptr);   // test2: stopping test 2
 int pcg_loop_f(const PcgDevF& F, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init = nullptr);
 
-void launch_slayer_h(const Dev& d, cudaStream_t st);
-void launch_vel(const Dev& d, const int* ce, int nce, const int* cn, int ncn, cudaStream_t st);
-void launch_exsal_imsal(const Dev& d, const Tune& tu, cudaStream_t st);
+// full: every layer as the reference; else only what fd's later stages do not write or read elsewhere
+void launch_slayer_h(const Dev& d, bool full, cudaStream_t st);
+void launch_vel(const Dev& d, cudaStream_t st);
+// h_from_hp: h was left unwritten below the surface layers (the short form of launch_slayer_h)
+void launch_exsal_imsal(const Dev& d, const Tune& tu, bool h_from_hp, cudaStream_t st);
 // Non-active tracers (k_tracer.cu): exTracer + ImTracer for ntr tracers at once.  Tracer nt
 // (0-based) of a pool is the layer-major field at pool + nt * stride.  `cpp` holds tracerpp, `tr`
 // receives tracer; layers without a solve keep the tracer pool's values, or tracerpp's when

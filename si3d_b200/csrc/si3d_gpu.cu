@@ -78,10 +78,7 @@ struct Ctx {
   si3d_params prm{};
   int lm = 0, lm1 = 0, km1 = 0, P = 0;
   std::vector<void*> allocs;
-  // face-column lists (id_columnCE / id_columnCN)
-  int* ce = nullptr;
-  int* cn = nullptr;
-  int nce = 0, ncn = 0;
+  int nce = 0, ncn = 0;      // face columns (id_columnCE / id_columnCN)
   FaceMeta* mce = nullptr;   // static indices of the u / v face columns (momentum stage)
   FaceMeta* mcn = nullptr;
   MomTiles tce, tcn;         // their tiles (fused momentum kernel)
@@ -1129,11 +1126,11 @@ void obc_continuity(Ctx* c) {
   for (const ObcDev& b : c->obc) obc_vel(c->d, b, c->st);   // MODvel4openBC (:2821)
 }
 void vel_stage(Ctx* c) {
-  launch_vel(c->d, c->ce, c->nce, c->cn, c->ncn, c->st);
+  launch_vel(c->d, c->st);
   obc_continuity(c);
 }
-int scalar_stage(Ctx* c) {
-  launch_exsal_imsal(c->d, c->tune, c->st);
+int scalar_stage(Ctx* c, bool h_from_hp) {
+  launch_exsal_imsal(c->d, c->tune, h_from_hp, c->st);
   for (size_t b = 0; b < c->obc.size(); ++b) {   // openbcSCA (:515)
     const double v = series_at(c->obc_tmp[b], c->thrs, c->obc_dtsec / 3600.);
     if (std::isnan(v)) return SI3D_EDIMS;
@@ -1166,13 +1163,15 @@ int fd_pre(Ctx* c, int istep) {
 // fd after the zeta solve: surface layer, openbcUVH, velocities, scalar, tracers, wetting, mixing.
 int fd_post(Ctx* c, bool lastiter) {
   Dev& d = c->d;
-  int rc = stage(c, ST_SLAYER, 1, [&] { launch_slayer_h(d, c->st); });
+  // (the tracers read h itself below the surface)
+  const bool full = c->prm.ntr > 0 && c->prm.niter > 0 && lastiter;
+  int rc = stage(c, ST_SLAYER, 1, [&] { launch_slayer_h(d, full, c->st); });
   if (!rc) rc = obc_uvh(c);   // openbcUVH after the solve (:482)
   if (!rc) c->launches += obc_launches(c);
   if (!rc) rc = stage(c, ST_VEL, 3 + obc_launches(c), [&] { vel_stage(c); });
   if (!rc && c->prm.isal != 0) {
     int rs = 0;
-    rc = stage(c, ST_SCALAR, 3 + obc_launches(c), [&] { rs = scalar_stage(c); });
+    rc = stage(c, ST_SCALAR, 3 + obc_launches(c), [&] { rs = scalar_stage(c, !full); });
     if (!rc) rc = rs;
   }
   if (!rc && c->prm.ntr > 0 && c->prm.niter > 0 && lastiter)
@@ -1304,6 +1303,16 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
   d.g.lNC = up_int(g->lNC, lm, lm1);
   d.g.lSC = up_int(g->lSC, lm, lm1);
   d.g.kmz = up_int(g->kmz, lm1, km1);
+  {
+    std::vector<int> ku(lm), kv(lm);
+    for (int l = 0; l < lm; ++l) {
+      const int e = g->lEC[l], n = g->lNC[l];
+      ku[l] = e == lm1 ? 0 : std::min(g->kmz[l], g->kmz[e - 1]);
+      kv[l] = n == lm1 ? 0 : std::min(g->kmz[l], g->kmz[n - 1]);
+    }
+    d.g.kmu = up_int(ku.data(), lm, 0);
+    d.g.kmv = up_int(kv.data(), lm, 0);
+  }
   d.g.hhs = up_dbl(g->hhs, lm1);
   d.g.hhu = up_dbl(g->hhu, lm1);
   d.g.hhv = up_dbl(g->hhv, lm1);
@@ -1393,11 +1402,6 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
     if (g->lNC[l - 1] != lm1) cn.push_back(l);
   }
   c->nce = (int)ce.size(); c->ncn = (int)cn.size();
-  rc |= c->alloc(&c->ce, ce.size());
-  rc |= c->alloc(&c->cn, cn.size());
-  if (rc) { delete c; return rc; }
-  if (!ce.empty()) cudaMemcpy(c->ce, ce.data(), ce.size() * sizeof(int), cudaMemcpyHostToDevice);
-  if (!cn.empty()) cudaMemcpy(c->cn, cn.data(), cn.size() * sizeof(int), cudaMemcpyHostToDevice);
   {
     // static per-face indices of the momentum stage (exmom/matmom neighbours and layer bounds)
     auto kz = [&](int q) { return g->kmz[q - 1]; };
@@ -1447,7 +1451,9 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
     // Before the autotuner: the fused momentum kernel once its tiles give every SM one, else the split
     // kernels, whose cells spread over all SMs (both directions of one call, split / fused: 31 tiles
     // 75 / 81 us, 800 tiles 195 / 166 us, 1260 tiles 442 / 340 us)
-    if (c->tce.ntile < pr.multiProcessorCount) { c->tune.mom_cl = 8; c->tune.mom_nt = 64; }
+    // and the scalar kernels with as many lanes as fill the chip (31 tiles 8 lanes 28, 4 lanes 30 us;
+    // 800 tiles 79 and 69 us)
+    if (c->tce.ntile < pr.multiProcessorCount) { c->tune.mom_cl = 8; c->tune.mom_nt = 64; c->tune.sal_cl = 8; c->tune.sal_nt = 128; }
   }
   rc = build_pcg(c, g);
   if (!rc) rc = c->alloc(&c->hist, (size_t)kHistSlots * (c->pcg.R.n + c->pcg.B.n + 2));
@@ -1746,9 +1752,9 @@ int si3d_gpu_stage(int h, const char* stage, int istep, si3d_step_stats* st) {
     if (rc) return rc;
     if (st) { st->nsolves = 1; st->iters[0] = it; st->relres[0] = rr; st->ier[0] = ier; st->total_iters = it; }
     if (ier < 0) return ier;
-    launch_slayer_h(d, c->st);
+    launch_slayer_h(d, true, c->st);
   } else if (s == "vel") vel_stage(c);
-  else if (s == "scalar") { if (int rc = scalar_stage(c)) return rc; }
+  else if (s == "scalar") { if (int rc = scalar_stage(c, false)) return rc; }
   else if (s == "tracer") { if (c->prm.ntr > 0) tracer_stage(c); }
   else if (s == "turbulence") { if (c->prm.iturb == 1) launch_turbulence(d, c->turb_scr, c->st); }
   else if (s == "vel2") launch_vel2(d, c->st);
@@ -1959,7 +1965,7 @@ static int time_stage(Ctx* c, int which, int reps, float* best) {
       momentum_stage(c, 1);
       momentum_stage(c, 2);
     } else {
-      launch_exsal_imsal(d, c->tune, c->st);
+      launch_exsal_imsal(d, c->tune, false, c->st);
     }
   };
   run();   // warm-up
