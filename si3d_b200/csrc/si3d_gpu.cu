@@ -96,11 +96,10 @@ struct Ctx {
   double obc_dtsec = 0, thrs = 0;
   MgDev mg{};                // aggregation hierarchy of the MG inner solves (precision SI3D_MIXED_MG)
   int mg_blocks = 0;
-  PcgScal* h_scf = nullptr;  // pinned
+  PcgScal* h_scf = nullptr;  // behind h_sc
   int last_inner = 8;
   long long ir_outer = 0;
   PcgScal* h_sc = nullptr;  // pinned
-  double* h_hist = nullptr; // pinned, 2 x itmax
   int last_iters = 8;
   // whole-solve cooperative kernel (k_pcg_persistent.cu); false -> one launch per phase
   bool persistent = true;
@@ -196,25 +195,46 @@ struct Ctx {
       if (e) cudaEventDestroy(e);
     for (void* p : allocs) cudaFree(p);
     if (h_sc) cudaFreeHost(h_sc);
-    if (h_scf) cudaFreeHost(h_scf);
-    if (h_hist) cudaFreeHost(h_hist);
     if (cst) cudaStreamSynchronize(cst);
     for (cudaEvent_t e : {ev0, ev1, evp0, evp1, pe0, pe1, out_packed, out_free[0], out_free[1]}) if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : out_done) if (e) cudaEventDestroy(e);
     if (cst) cudaStreamDestroy(cst);
     if (st) cudaStreamDestroy(st);
   }
-  template <class T>
-  int alloc(T** p, size_t n) {
-    void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(T));
+  // Zeroed device memory that lives as long as the handle.  Arrays up to kSlabItem bytes share slabs: a
+  // handle has about a hundred of them, and an allocation with its zero fill and synchronisation (and
+  // the free at the end) costs 0.1 to 0.2 ms each (the stand-alone zeta solve of 52500 columns, which
+  // makes and drops a handle: 34 ms with one allocation per array).
+  static constexpr size_t kSlabItem = 4 << 20, kSlab = 32 << 20;
+  char* slab = nullptr;
+  size_t slab_left = 0;
+  int fresh(void** q, size_t bytes) {
+    cudaError_t e = cudaMalloc(q, bytes);
     if (e != cudaSuccess) { g_last_cuda = cudaGetErrorString(e); return SI3D_ENOMEM; }
-    allocs.push_back(q);
+    allocs.push_back(*q);
     // the zero fill runs on the legacy default stream, which the handle's non-blocking streams do
     // not wait for: finish it before the buffer is handed out
-    e = cudaMemset(q, 0, std::max<size_t>(n, 1) * sizeof(T));
+    e = cudaMemset(*q, 0, bytes);
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e != cudaSuccess) { g_last_cuda = cudaGetErrorString(e); return SI3D_ECUDA; }
+    return 0;
+  }
+  template <class T>
+  int alloc(T** p, size_t n) {
+    const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;   // cudaMalloc's alignment
+    void* q = nullptr;
+    if (bytes > kSlabItem) {
+      if (int rc = fresh(&q, bytes)) return rc;
+    } else {
+      if (slab_left < bytes) {
+        if (int rc = fresh(&q, kSlab)) return rc;
+        slab = static_cast<char*>(q);
+        slab_left = kSlab;
+      }
+      q = slab;
+      slab += bytes;
+      slab_left -= bytes;
+    }
     *p = static_cast<T*>(q);
     return 0;
   }
@@ -698,8 +718,8 @@ int build_pcg(Ctx* c, const si3d_grid* g) {
   rc |= c->alloc(&P.hist_beta, cap);
   rc |= c->alloc(&P.tri, 2 * (size_t)(cap + 1));
   if (rc) return rc;
-  CK(cudaMallocHost(&c->h_sc, sizeof(PcgScal)));
-  CK(cudaMallocHost(&c->h_hist, sizeof(double) * 2 * cap));
+  CK(cudaMallocHost(&c->h_sc, 2 * sizeof(PcgScal)));   // the FP64 scalars, then the inner solves'
+  c->h_scf = c->h_sc + 1;
   // FP32 copy of the system for the inner solves of iterative refinement (shares the node lists,
   // neighbour indices and reduction buffers with the FP64 system)
   PcgDevF& F = c->pcgf;
@@ -714,7 +734,6 @@ int build_pcg(Ctx* c, const si3d_grid* g) {
   if (rc) return rc;
   F.part0 = P.part0; F.part1 = P.part1; F.part2 = P.part2; F.part3 = P.part3; F.part_n = P.part_n;
   F.hist_alpha = P.hist_alpha; F.hist_beta = P.hist_beta; F.tri = nullptr;
-  CK(cudaMallocHost(&c->h_scf, sizeof(PcgScal)));
   if (c->prm.precision == SI3D_MIXED_MG) return build_mg(c, g);
   if (c->prm.ordering == SI3D_ORDER_NATURAL) return build_natural(c, g);
   return 0;
@@ -1238,7 +1257,9 @@ const char* si3d_gpu_strerror(int code) {
   }
 }
 
-int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* handle) {
+// solver_only: the zeta system alone (si3d_gpu_solve_zeta), without the 3-D state and what the other
+// stages need.
+static int init_handle(const si3d_grid* g, const si3d_params* prm, int device, bool solver_only, int* handle) {
   if (!g || !prm || !handle) return SI3D_EDIMS;
   if (g->lm < 1 || g->km1 < 3 || g->km1 > SI3D_MAXK || g->k1 != 2) return SI3D_EDIMS;
   if (prm->itrmom != 1 || prm->ihd > 1 || prm->pcg_itmax < 1 || (prm->pcg_test != 5 && prm->pcg_test != 2))
@@ -1262,9 +1283,10 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
     return SI3D_EDIMS;
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= device) return SI3D_ENODEV;
-  cudaDeviceProp pr;
-  CK(cudaGetDeviceProperties(&pr, device));
-  if (pr.major < 10) return SI3D_ENODEV;
+  int major = 0, sms = 0;
+  CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, device));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+  if (major < 10) return SI3D_ENODEV;
   CK(cudaSetDevice(device));
   Ctx* c = new Ctx();
   c->device = device;
@@ -1336,7 +1358,7 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
   // state
   const size_t n3 = (size_t)km1 * P;
   Fields3& f = d.f;
-  for (double** q : {&f.uh, &f.uhp, &f.uhpp, &f.up, &f.upp, &f.hu, &f.hup, &f.hupp, &f.agx, &f.arx, &f.vh, &f.vhp,
+  if (!solver_only) for (double** q : {&f.uh, &f.uhp, &f.uhpp, &f.up, &f.upp, &f.hu, &f.hup, &f.hupp, &f.agx, &f.arx, &f.vh, &f.vhp,
                      &f.vhpp, &f.vp, &f.vpp, &f.hv, &f.hvp, &f.hvpp, &f.agy, &f.ary, &f.h, &f.hp, &f.hpp, &f.sal,
                      &f.salp, &f.salpp, &f.rhop, &f.Av, &f.Dv, &f.wp, &f.HeatSource, &f.Bth2, &f.Bth3, &f.Bth4})
     rc |= c->alloc(q, n3);
@@ -1345,6 +1367,7 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
                      &s.uair, &s.vair, &s.cdw, &s.rsx, &s.rsy})
     rc |= c->alloc(q, P);
   for (int** q : {&s.k1z, &s.k1u, &s.k1v}) rc |= c->alloc(q, P);
+  if (!solver_only) {
   rc |= c->alloc(&d.scr, n3);
   if (prm->iturb == 1) {
     for (double** q : {&f.q2, &f.q2p, &f.q2pp, &f.q2l, &f.q2lp, &f.q2lpp, &f.u, &f.v}) rc |= c->alloc(q, n3);
@@ -1372,9 +1395,11 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
     rc |= c->alloc(&c->tr_fx, n3 * 3 * std::min(std::max(prm->ntr - 1, 1), kTracerFluxGroup));
   }
   rc |= c->alloc(&c->staging, (size_t)km1 * lm1);
+  }
   rc |= c->alloc(&c->dz, P);
   rc |= c->alloc(&c->d_stats_ii, 48);
   rc |= c->alloc(&c->d_stats_rr, 24);
+  if (!solver_only) {
   if (!rc && momentum_init(km1) != 0) { g_last_cuda = "momentum kernel shared-memory attribute"; rc = SI3D_ECUDA; }
   if (!rc && transport_init(km1) != 0) { g_last_cuda = "continuity kernel shared-memory attribute"; rc = SI3D_ECUDA; }
   // pixel (i - 1) * jm1 + (j - 1) of every wet column in the (im1, jm1) image of the learned
@@ -1453,8 +1478,10 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
     // 75 / 81 us, 800 tiles 195 / 166 us, 1260 tiles 442 / 340 us)
     // and the scalar kernels with as many lanes as fill the chip (31 tiles 8 lanes 28, 4 lanes 30 us;
     // 800 tiles 79 and 69 us)
-    if (c->tce.ntile < pr.multiProcessorCount) { c->tune.mom_cl = 8; c->tune.mom_nt = 64; c->tune.sal_cl = 8; c->tune.sal_nt = 128; }
+    if (c->tce.ntile < sms) { c->tune.mom_cl = 8; c->tune.mom_nt = 64; c->tune.sal_cl = 8; c->tune.sal_nt = 128; }
   }
+  }
+  if (rc) { delete c; return rc; }
   rc = build_pcg(c, g);
   if (!rc) rc = c->alloc(&c->hist, (size_t)kHistSlots * (c->pcg.R.n + c->pcg.B.n + 2));
   if (rc) { delete c; return rc; }
@@ -1463,6 +1490,10 @@ int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* h
   g_ctx.push_back(c);
   *handle = (int)g_ctx.size() - 1;
   return 0;
+}
+
+int si3d_gpu_init(const si3d_grid* g, const si3d_params* prm, int device, int* handle) {
+  return init_handle(g, prm, device, false, handle);
 }
 
 void si3d_gpu_finalize(int h) {
@@ -2723,7 +2754,7 @@ int si3d_gpu_solve_zeta(int lm, const double* coef, const int* jcoef, const doub
   prm.ordering = ordering == SI3D_ORDER_NATURAL ? SI3D_ORDER_NATURAL : SI3D_ORDER_REDBLACK;
   prm.x0_mode = SI3D_X0_PREV; prm.precision = precision;
   int hdl = -1;
-  int rc = si3d_gpu_init(&g, &prm, 0, &hdl);
+  int rc = init_handle(&g, &prm, 0, true, &hdl);
   if (rc) return rc;
   Ctx* c = get(hdl);
   int ier = 0, it = 0;
