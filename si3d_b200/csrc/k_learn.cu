@@ -42,19 +42,6 @@ constexpr int WG_BLOCKS = 296;                 // weight-gradient partial sums (
 
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
-struct TileIdx {
-  int b, i0, j0;
-};
-__device__ __forceinline__ TileIdx tile_of(int t, int H, int W) {
-  const int nj = (W + TW - 1) / TW, ni = (H + TH - 1) / TH;
-  TileIdx r;
-  r.b = t / (ni * nj);
-  const int rem = t % (ni * nj);
-  r.i0 = (rem / nj) * TH;
-  r.j0 = (rem % nj) * TW;
-  return r;
-}
-
 // ------------------------------------------------------------------ weights
 // Block weights to the tensor-core layout [tap][n][k] (bf16): forward n = cout, k = cin;
 // data gradient n = cin, k = cout with the tap mirrored.  Stem/head weights rounded to bf16 values.
@@ -157,18 +144,19 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
       : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-enum { CONV_FWD = 0, CONV_BWD = 1 };
+// Behind a layer's G (the gradient of its input x_k): DY = G * (y_k > 0), the gradient at the ReLU of
+// the layer below, in FP32 for the weight gradient and (unless it is the stem's) in BF16 for the
+// tensor-core data gradient.  Written by the kernel that makes G, which spares a pass over G a layer
+// (32 x 64 x 64 pixels: five passes of 19.5 us; the data gradient takes 32.6 instead of 25.5 us).
+__device__ __forceinline__ float relu_grad(float g, float y) { return y > 0.f ? g : 0.f; }
 
-// out[p][n] = sum_{tap, k} in[p + off(tap)][k] * Wk[tap][n][k].
-// CONV_FWD: y = out + bias; X_out = bf16(X_in + ReLU(y)); Y (optional) = y.
-// CONV_BWD: G_out = G_in + out.
-// Persistent blocks: the weights go to shared memory once per block, which then loops over 8 x 16
-// pixel tiles (tile = blockIdx.x, blockIdx.x + gridDim.x, ...).
-template <int MODE>
-__global__ void __launch_bounds__(128) k_conv32(const bf16* __restrict__ Xin, const bf16* __restrict__ Wk,
-                                                const float* __restrict__ bias, int B, int H, int W,
-                                                bf16* __restrict__ Xout, float* __restrict__ Y,
-                                                const float* __restrict__ Gin, float* __restrict__ Gout) {
+// Data gradient of a 32 -> 32 layer: G[p][n] += sum_{tap, k} in[p + off(tap)][k] * Wk[tap][n][k], in place
+// (a thread reads and writes the same elements), and for the layer below DY and (not for the stem) DYb
+// from its y.  Persistent blocks: the weights go to shared memory once per block, which then loops over
+// 8 x 16 pixel tiles (tile = blockIdx.x, blockIdx.x + gridDim.x, ...).
+__global__ void __launch_bounds__(128) k_conv32_bwd(const bf16* __restrict__ Xin, const bf16* __restrict__ Wk, int B,
+                                                    int H, int W, float* __restrict__ G, const float* __restrict__ Y,
+                                                    float* __restrict__ DY, bf16* __restrict__ DYb) {
   __shared__ __align__(16) bf16 sX[HT * WT * XS];
   __shared__ __align__(16) bf16 sW[9 * C * XS];
   for (int r = threadIdx.x; r < 9 * C * 4; r += 128) {
@@ -232,18 +220,14 @@ __global__ void __launch_bounds__(128) k_conv32(const bf16* __restrict__ Xin, co
         const size_t p = ((size_t)b * H + gi) * W + gj;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-          const int co = nt * 8 + 2 * q;
-          const float v0 = acc[r][nt][2 * half], v1 = acc[r][nt][2 * half + 1];
-          if (MODE == CONV_FWD) {
-            const float y0 = v0 + bias[co], y1 = v1 + bias[co + 1];
-            const bf16* xc = &sX[((ty + 1) * WT + tj + 1) * XS + co];
-            const float x0 = __bfloat162float(xc[0]), x1 = __bfloat162float(xc[1]);
-            if (Y) *reinterpret_cast<float2*>(Y + p * C + co) = make_float2(y0, y1);
-            *reinterpret_cast<__nv_bfloat162*>(Xout + p * C + co) =
-                __floats2bfloat162_rn(x0 + fmaxf(y0, 0.f), x1 + fmaxf(y1, 0.f));
-          } else {
-            const float2 gi2 = *reinterpret_cast<const float2*>(Gin + p * C + co);
-            *reinterpret_cast<float2*>(Gout + p * C + co) = make_float2(gi2.x + v0, gi2.y + v1);
+          const size_t o = p * C + nt * 8 + 2 * q;
+          const float2 gi2 = *reinterpret_cast<const float2*>(G + o), y = *reinterpret_cast<const float2*>(Y + o);
+          const float2 go = make_float2(gi2.x + acc[r][nt][2 * half], gi2.y + acc[r][nt][2 * half + 1]);
+          const float2 d = make_float2(relu_grad(go.x, y.x), relu_grad(go.y, y.y));
+          *reinterpret_cast<float2*>(DY + o) = d;
+          if (DYb) {
+            *reinterpret_cast<float2*>(G + o) = go;
+            *reinterpret_cast<__nv_bfloat162*>(DYb + o) = __floats2bfloat162_rn(d.x, d.y);
           }
         }
       }
@@ -577,114 +561,232 @@ __global__ void __launch_bounds__(TP) k_head(const bf16* __restrict__ X, const f
 }
 
 // ------------------------------------------------------------------ backward pieces
-// G4[p][ci] = sum_tap gout[p - off(tap)] * wh[tap][ci]
+// G4[p][ci] = sum_tap gout[p - off(tap)] * wh[tap][ci], and DY, DYb from it.  A thread has four channels
+// of a pixel, so that a warp writes whole lines (29 -> 15 us at 32 x 64 x 64, the ReLU's pass included).
 __global__ void __launch_bounds__(TP) k_head_bwd(const float* __restrict__ gout, const float* __restrict__ w, int H,
-                                                 int W, float* __restrict__ G) {
+                                                 int W, const float* __restrict__ Y, float* __restrict__ G,
+                                                 float* __restrict__ DY, bf16* __restrict__ DYb) {
   __shared__ float sG[HT * WT];
-  __shared__ float sW[9 * C];
   const int b = blockIdx.z, i0 = blockIdx.y * TH, j0 = blockIdx.x * TW;
-  for (int r = threadIdx.x; r < 9 * C; r += TP) sW[r] = w[r];
+  const int c4 = (threadIdx.x % (C / 4)) * 4;
+  float wr[9][4];
+#pragma unroll
+  for (int t = 0; t < 9; ++t)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) wr[t][e] = w[t * C + c4 + e];
   for (int r = threadIdx.x; r < HT * WT; r += TP) {
     const int gi = i0 + r / WT - 1, gj = j0 + r % WT - 1;
     sG[r] = (gi >= 0 && gi < H && gj >= 0 && gj < W) ? gout[((size_t)b * H + gi) * W + gj] : 0.f;
   }
   __syncthreads();
-  const int ti = threadIdx.x / TW, tj = threadIdx.x % TW;
-  const int gi = i0 + ti, gj = j0 + tj;
-  if (gi >= H || gj >= W) return;
-  const size_t p = ((size_t)b * H + gi) * W + gj;
-  for (int ci = 0; ci < C; ++ci) {
-    float acc = 0.f;
+#pragma unroll 4
+  for (int pix = threadIdx.x / (C / 4); pix < TP; pix += TP / (C / 4)) {
+    const int ti = pix / TW, tj = pix % TW, gi = i0 + ti, gj = j0 + tj;
+    if (gi >= H || gj >= W) continue;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
     for (int t = 0; t < 9; ++t) {
       const int tm = 8 - t;   // gout at p + off(8 - t) = p - off(t)
-      acc = acc + sG[(ti + 1 + tm / 3 - 1) * WT + tj + 1 + tm % 3 - 1] * sW[t * C + ci];
+      const float g = sG[(ti + tm / 3) * WT + tj + tm % 3];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[e] = acc[e] + g * wr[t][e];
     }
-    G[p * C + ci] = acc;
+    const size_t o = (((size_t)b * H + gi) * W + gj) * C + c4;
+    const float4 y = *reinterpret_cast<const float4*>(Y + o);
+    const float4 d = make_float4(relu_grad(acc[0], y.x), relu_grad(acc[1], y.y), relu_grad(acc[2], y.z), relu_grad(acc[3], y.w));
+    *reinterpret_cast<float4*>(G + o) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    *reinterpret_cast<float4*>(DY + o) = d;
+    *reinterpret_cast<__nv_bfloat162*>(DYb + o) = __floats2bfloat162_rn(d.x, d.y);
+    *reinterpret_cast<__nv_bfloat162*>(DYb + o + 2) = __floats2bfloat162_rn(d.z, d.w);
   }
 }
 
-// DY = G * (Y > 0) in FP32 and a BF16 copy for the tensor-core data gradient.
-__global__ void k_relu_bwd(const float* __restrict__ G, const float* __restrict__ Y, float* __restrict__ DY,
-                           bf16* __restrict__ DYb, size_t n) {
-  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float v = Y[i] > 0.f ? G[i] : 0.f;
-  DY[i] = v;
-  if (DYb) DYb[i] = __float2bfloat16_rn(v);
-}
-
-template <typename XT>
-__device__ __forceinline__ float ld_as_float(const XT* p);
-template <>
-__device__ __forceinline__ float ld_as_float<float>(const float* p) { return bfr(*p); }
-template <>
-__device__ __forceinline__ float ld_as_float<bf16>(const bf16* p) { return __bfloat162float(*p); }
-
 // Weight gradient partials: part[blk][(tap * CIN + ci) * COUT + co] = sum over the block's tiles of
-// X[p + off(tap)][ci] * DY[p][co], and part[blk][9 * CIN * COUT + co] = sum DY[p][co].  Thread
-// (rg, co) owns output channel co and the (tap, ci) rows rg, rg + NRG, ...; pixels are the outer loop,
-// so each step reads one DY value and broadcasts X across the warp.
+// X[p + off(tap)][ci] * DY[p][co], and part[blk][9 * CIN * COUT + co] = sum DY[p][co].  FP32 on the FP32
+// cores (DY is held in FP32).  A tile's X (one pixel of frame) and DY are staged in shared memory, and a
+// thread walks the tile's pixels row by row with the 3 x 3 window of X in registers, so a pixel costs
+// three loads of X whatever the number of taps.  What a lane and a warp own depends on the layer:
+//   32 -> 32  lane = ci, warp = four co: 9 x 4 sums a thread, all pixels (40 instructions for 36 FMA)
+//    4 -> 32  lane = co, four ci a thread (one 16-byte load of X): 36 sums, the warps share the rows
+//   32 -> 1   lane = ci: 9 sums, the warps share the rows
+// The warps that share rows add their sums at the end in a fixed order.  The next
+// tile's values are fetched into registers behind the tile's arithmetic.  32 x 64 x 64 pixels, per call,
+// with one load of X per multiply-add and no FMA -> this: 200 -> 66, 57 -> 16 and 63 -> 11 us (8 x 16
+// pixel tiles without the fetch ahead: 94, 29, 44).
+constexpr int WGW = 8;                     // warps of a weight-gradient block
+constexpr int GH = 4, GP = GH * TW;        // its tiles: 4 x 16 pixels
+constexpr int GHP = (GH + 2) * WT;         // with halo
 template <int CIN, int COUT, typename XT>
-__global__ void __launch_bounds__(256) k_wgrad(const XT* __restrict__ X, const float* __restrict__ DY, int B, int H,
-                                               int W, float* __restrict__ part) {
-  constexpr int R = 9 * CIN;
-  constexpr int NRG = 256 / COUT;
-  constexpr int PER = (R + NRG - 1) / NRG;
-  constexpr int NOUT = R * COUT + COUT;
-  __shared__ float sX[HT * WT * CIN];
-  __shared__ float sD[TP * COUT];
-  const int co = threadIdx.x % COUT, rg = threadIdx.x / COUT;
-  float acc[PER];
-  float accb = 0.f;
+__global__ void __launch_bounds__(32 * WGW, 2) k_wgrad(const XT* __restrict__ X, const float* __restrict__ DY, int B,
+                                                       int H, int W, float* __restrict__ part) {
+  constexpr bool FULL = CIN == 32 && COUT == 32;   // the three shapes of the network
+  constexpr bool STEM = CIN == 4 && COUT == 32;
+  static_assert(FULL || STEM || (CIN == 32 && COUT == 1), "layer shape");
+  constexpr int NTH = 32 * WGW;
+  constexpr int R = 9 * CIN, NOUT = R * COUT + COUT;
+  constexpr int NQ = FULL || STEM ? 4 : 1;   // FULL: values of DY a window value meets; STEM: channels of a window pixel
+  constexpr int NX = STEM ? 4 : 1, ND = FULL ? 4 : 1;
+  constexpr int XV = CIN == 32 ? 8 : 1, NXL = (GHP * CIN / XV + NTH - 1) / NTH;     // loads of X a thread, values each
+  constexpr int DV = COUT == 32 ? 4 : 1, NDL = (GP * COUT / DV + NTH - 1) / NTH;    // of DY
+  __shared__ __align__(16) float sX[GHP * CIN];
+  __shared__ __align__(16) float sD[GP * COUT];
+  const int ln = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int nj = (W + TW - 1) / TW, ni = (H + GH - 1) / GH, ntiles = B * ni * nj;
+  float acc[9][NQ], accb[ND];
 #pragma unroll
-  for (int m = 0; m < PER; ++m) acc[m] = 0.f;
-  const int ntiles = B * ((H + TH - 1) / TH) * ((W + TW - 1) / TW);
+  for (int q = 0; q < ND; ++q) accb[q] = 0.f;
+#pragma unroll
+  for (int q = 0; q < NQ; ++q)
+#pragma unroll
+    for (int t = 0; t < 9; ++t) acc[t][q] = 0.f;
+  uint4 rx[CIN == 32 ? NXL : 1];
+  float rxf[CIN == 32 ? 1 : NXL];
+  float4 rd[COUT == 32 ? NDL : 1];
+  float rdf = 0.f;
+  auto fetch = [&](int tile) {   // a tile's X (zero outside the image) and DY to registers
+    const int b = tile / (ni * nj), rem = tile - b * (ni * nj), i0 = rem / nj * GH, j0 = rem % nj * TW;
+#pragma unroll
+    for (int k = 0; k < NXL; ++k) {
+      const int r = threadIdx.x + k * NTH, pix = r / (CIN / XV), c = r % (CIN / XV) * XV;
+      const int gi = i0 + pix / WT - 1, gj = j0 + pix % WT - 1;
+      const bool in = pix < GHP && gi >= 0 && gi < H && gj >= 0 && gj < W;
+      const size_t o = (((size_t)b * H + gi) * W + gj) * CIN + c;
+      if constexpr (CIN == 32) {
+        rx[k] = make_uint4(0u, 0u, 0u, 0u);
+        if (in) rx[k] = *reinterpret_cast<const uint4*>(X + o);
+      } else {
+        rxf[k] = in ? bfr(X[o]) : 0.f;
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NDL; ++k) {
+      const int r = threadIdx.x + k * NTH, pix = r / (COUT / DV), c = r % (COUT / DV) * DV;
+      const int gi = i0 + pix / TW, gj = j0 + pix % TW;
+      const bool in = pix < GP && gi < H && gj < W;
+      const size_t o = (((size_t)b * H + gi) * W + gj) * COUT + c;
+      if constexpr (COUT == 32) {
+        rd[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (in) rd[k] = *reinterpret_cast<const float4*>(DY + o);
+      } else {
+        rdf = in ? DY[o] : 0.f;
+      }
+    }
+  };
+  if ((int)blockIdx.x < ntiles) fetch(blockIdx.x);
   for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const TileIdx T = tile_of(tile, H, W);
     __syncthreads();
-    for (int r = threadIdx.x; r < HT * WT * CIN; r += 256) {
-      const int pix = r / CIN, ci = r % CIN;
-      const int gi = T.i0 + pix / WT - 1, gj = T.j0 + pix % WT - 1;
-      sX[r] = (gi >= 0 && gi < H && gj >= 0 && gj < W) ? ld_as_float<XT>(X + (((size_t)T.b * H + gi) * W + gj) * CIN + ci)
-                                                       : 0.f;
-    }
-    for (int r = threadIdx.x; r < TP * COUT; r += 256) {
-      const int pix = r / COUT, c = r % COUT;
-      const int gi = T.i0 + pix / TW, gj = T.j0 + pix % TW;
-      sD[r] = (gi < H && gj < W) ? DY[(((size_t)T.b * H + gi) * W + gj) * COUT + c] : 0.f;
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int pix = 0; pix < TP; ++pix) {
-      const float dv = sD[pix * COUT + co];
-      const int base = ((pix / TW) * WT + pix % TW) * CIN;
-      if (rg == 0) accb = accb + dv;
 #pragma unroll
-      for (int m = 0; m < PER; ++m) {
-        const int r = rg + NRG * m;
-        if (r < R) {
-          const int t = r / CIN, ci = r % CIN;
-          acc[m] = acc[m] + sX[base + ((t / 3) * WT + t % 3) * CIN + ci] * dv;
+    for (int k = 0; k < NXL; ++k) {
+      const int r = threadIdx.x + k * NTH;
+      if (r * XV < GHP * CIN) {
+        if constexpr (CIN == 32) {
+          const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&rx[k]);
+          const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
+          const float2 c = __bfloat1622float2(h[2]), d = __bfloat1622float2(h[3]);
+          *reinterpret_cast<float4*>(&sX[r * 8]) = make_float4(a.x, a.y, b.x, b.y);
+          *reinterpret_cast<float4*>(&sX[r * 8 + 4]) = make_float4(c.x, c.y, d.x, d.y);
+        } else {
+          sX[r] = rxf[k];
         }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < NDL; ++k) {
+      const int r = threadIdx.x + k * NTH;
+      if (r * DV < GP * COUT) {
+        if constexpr (COUT == 32) *reinterpret_cast<float4*>(&sD[r * 4]) = rd[k];
+        else sD[r] = rdf;
+      }
+    }
+    __syncthreads();
+    if (tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x);   // lands behind this tile's arithmetic
+    // FULL: every warp walks all rows; the others: half a row a warp
+    constexpr int LEN = FULL ? TW : TW / 2;
+    static_assert(FULL || WGW == 2 * GH, "half a row a warp");
+    for (int u = FULL ? 0 : wp; u < (FULL ? GH : wp + 1); ++u) {
+      const int ti = FULL ? u : u >> 1, t0 = FULL ? 0 : (u & 1) * LEN;
+      float x[3][3][NX];   // the 3 x 3 window of X (STEM: four channels of each)
+      auto column = [&](int c, int tj) {   // window column c from image column tj - 1
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+          const int o = ((ti + i) * WT + tj) * CIN;
+          if constexpr (STEM) {
+            const float4 v = *reinterpret_cast<const float4*>(&sX[o]);
+            x[i][c][0] = v.x; x[i][c][1] = v.y; x[i][c][2] = v.z; x[i][c][3] = v.w;
+          } else {
+            x[i][c][0] = sX[o + ln];
+          }
+        }
+      };
+      column(0, t0);
+      column(1, t0 + 1);
+#pragma unroll 4
+      for (int tj = t0; tj < t0 + LEN; ++tj) {
+        column(2, tj + 2);
+        const float* dp = &sD[(ti * TW + tj) * COUT];
+        float d[ND];
+        if constexpr (FULL) {
+          const float4 v = *reinterpret_cast<const float4*>(dp + 4 * wp);
+          d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+        } else {
+          d[0] = dp[STEM ? ln : 0];
+        }
+#pragma unroll
+        for (int q = 0; q < ND; ++q) accb[q] = accb[q] + d[q];
+#pragma unroll
+        for (int t = 0; t < 9; ++t)
+#pragma unroll
+          for (int q = 0; q < NQ; ++q) acc[t][q] = fmaf(x[t / 3][t % 3][STEM ? q : 0], d[FULL ? q : 0], acc[t][q]);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+          for (int q = 0; q < NX; ++q) { x[i][0][q] = x[i][1][q]; x[i][1][q] = x[i][2][q]; }
       }
     }
   }
   float* o = part + (size_t)blockIdx.x * NOUT;
+  if constexpr (FULL) {
 #pragma unroll
-  for (int m = 0; m < PER; ++m) {
-    const int r = rg + NRG * m;
-    if (r < R) o[r * COUT + co] = acc[m];
+    for (int t = 0; t < 9; ++t)
+      *reinterpret_cast<float4*>(&o[(t * CIN + ln) * COUT + 4 * wp]) = make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]);
+    if (ln == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) o[R * COUT + 4 * wp + q] = accb[q];
+    }
+  } else {
+    // the warps' sums of each output, added warp by warp
+    constexpr int NA = 9 * NQ + 1;   // sums of a thread
+    __shared__ float sA[WGW][NA * 32];
+#pragma unroll
+    for (int m = 0; m < NA; ++m) sA[wp][m * 32 + ln] = m < 9 * NQ ? acc[m / NQ % 9][m % NQ] : accb[0];
+    __syncthreads();
+    for (int r = threadIdx.x; r < NA * 32; r += NTH) {
+      const int m = r >> 5, l = r & 31;
+      float v = sA[0][r];
+      for (int w = 1; w < WGW; ++w) v = v + sA[w][r];
+      if (m < 9 * NQ) o[STEM ? m * COUT + l : m * CIN + l] = v;   // m = tap (x 4 + ci)
+      else if (STEM || l == 0) o[R * COUT + l] = v;
+    }
   }
-  if (rg == 0) o[R * COUT + co] = accb;
 }
 
-// grad[off + o] = sum_blk part[blk][o] (fixed order); the weight part [9][CIN][COUT] first, then
-// the COUT bias entries.
-__global__ void k_wgrad_reduce(const float* __restrict__ part, int nblk, int nout, float* __restrict__ grad) {
-  const int o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= nout) return;
+// grad[off + o] = sum_blk part[blk][o] (fixed order: WR threads of an output each take every WR-th block,
+// then their sums in order); the weight part [9][CIN][COUT] first, then the COUT bias entries.  One
+// thread per output left three SMs in four idle (21 us for the 9248 outputs of a block, 8.6 so).
+constexpr int WR = 8;
+__global__ void __launch_bounds__(32 * WR) k_wgrad_reduce(const float* __restrict__ part, int nblk, int nout,
+                                                          float* __restrict__ grad) {
+  __shared__ float sh[WR][32];
+  const int o = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
-  for (int b = 0; b < nblk; ++b) s = s + part[(size_t)b * nout + o];
+  if (o < nout) {
+#pragma unroll 4
+    for (int b = threadIdx.y; b < nblk; b += WR) s = s + part[(size_t)b * nout + o];
+  }
+  sh[threadIdx.y][threadIdx.x] = s;
+  __syncthreads();
+  if (threadIdx.y != 0 || o >= nout) return;
+  for (int w = 1; w < WR; ++w) s = s + sh[w][threadIdx.x];
   grad[o] = s;
 }
 
@@ -827,8 +929,8 @@ size_t Workspace::bytes(int B, int H, int W, bool training) {
   for (int i = 0; i < nx; ++i) add(P * C * sizeof(bf16));
   if (training) {
     for (int i = 0; i < SI3D_NET_BLOCKS + 1; ++i) add(P * C * sizeof(float));   // y0..y4
-    for (int i = 0; i < 3; ++i) add(P * C * sizeof(float));                     // G, G', DY
-    add(P * C * sizeof(bf16));                                                   // DYb
+    for (int i = 0; i < 2; ++i) add(P * C * sizeof(float));                     // G, DY
+    for (int i = 0; i < 2; ++i) add(P * C * sizeof(bf16));                      // DYb of two layers
     add((size_t)WG_BLOCKS * (9 * C * C + C) * sizeof(float));                    // weight-gradient partials
   }
   return s;
@@ -847,15 +949,14 @@ bool Workspace::carve(void* base, size_t avail, int B, int H, int W, bool traini
   for (int i = 0; i < SI3D_NET_BLOCKS + 1; ++i) x[i] = nullptr;
   for (int i = 0; i < nx; ++i) x[i] = static_cast<bf16*>(take(P * C * sizeof(bf16)));
   for (int i = 0; i < SI3D_NET_BLOCKS + 1; ++i) y[i] = nullptr;
-  G0 = G1 = DY = nullptr;
-  DYb = nullptr;
+  G = DY = nullptr;
+  DYb[0] = DYb[1] = nullptr;
   part = nullptr;
   if (training) {
     for (int i = 0; i < SI3D_NET_BLOCKS + 1; ++i) y[i] = static_cast<float*>(take(P * C * sizeof(float)));
-    G0 = static_cast<float*>(take(P * C * sizeof(float)));
-    G1 = static_cast<float*>(take(P * C * sizeof(float)));
+    G = static_cast<float*>(take(P * C * sizeof(float)));
     DY = static_cast<float*>(take(P * C * sizeof(float)));
-    DYb = static_cast<bf16*>(take(P * C * sizeof(bf16)));
+    for (int i = 0; i < 2; ++i) DYb[i] = static_cast<bf16*>(take(P * C * sizeof(bf16)));
     part = static_cast<float*>(take((size_t)WG_BLOCKS * (9 * C * C + C) * sizeof(float)));
   }
   this->training = training;
@@ -868,12 +969,11 @@ void prepare(const Workspace& ws, const float* params, cudaStream_t st) {
 }
 
 // Persistent grid of the convolution: every resident block of the device, at most one per tile.
-template <int MODE>
-int conv_blocks(int B, int H, int W) {
+int conv_bwd_blocks(int B, int H, int W) {
   int dev = 0, sms = 1, occ = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_conv32<MODE>, 128, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_conv32_bwd, 128, 0);
   const long long ntiles = (long long)B * ((H + TH - 1) / TH) * ((W + TW - 1) / TW);
   return (int)std::max(1LL, std::min(ntiles, (long long)sms * std::max(occ, 1)));
 }
@@ -946,25 +1046,19 @@ int forward(const Workspace& ws, const float* params, const float* feat, int B, 
 void backward(const Workspace& ws, const float* feat, const float* gout, int B, int H, int W, float* grad,
               cudaStream_t st) {
   const dim3 grid = tiles(B, H, W);
-  const size_t n = (size_t)B * H * W * C;
-  const int eb = (int)((n + 255) / 256);
   // head
-  k_wgrad<C, 1, bf16><<<WG_BLOCKS, 256, 0, st>>>(ws.x[SI3D_NET_BLOCKS], gout, B, H, W, ws.part);
-  k_wgrad_reduce<<<(9 * C + 1 + 255) / 256, 256, 0, st>>>(ws.part, WG_BLOCKS, 9 * C + 1, grad + OFF_HEAD_W);
-  k_head_bwd<<<grid, TP, 0, st>>>(gout, ws.head, H, W, ws.G0);
-  float* G = ws.G0;
-  float* Gn = ws.G1;
-  for (int k = SI3D_NET_BLOCKS - 1; k >= 0; --k) {
-    k_relu_bwd<<<eb, 256, 0, st>>>(G, ws.y[k + 1], ws.DY, ws.DYb, n);
-    k_wgrad<C, C, bf16><<<WG_BLOCKS, 256, 0, st>>>(ws.x[k], ws.DY, B, H, W, ws.part);
-    k_wgrad_reduce<<<(BLK_SZ + 255) / 256, 256, 0, st>>>(ws.part, WG_BLOCKS, BLK_SZ, grad + OFF_BLK + k * BLK_SZ);
-    k_conv32<CONV_BWD><<<conv_blocks<CONV_BWD>(B, H, W), 128, 0, st>>>(ws.DYb, ws.wbwd + (size_t)k * 9 * C * C, nullptr,
-                                                                       B, H, W, nullptr, nullptr, G, Gn);
-    std::swap(G, Gn);
+  k_wgrad<C, 1, bf16><<<WG_BLOCKS, 32 * WGW, 0, st>>>(ws.x[SI3D_NET_BLOCKS], gout, B, H, W, ws.part);
+  k_wgrad_reduce<<<(9 * C + 1 + 31) / 32, dim3(32, WR), 0, st>>>(ws.part, WG_BLOCKS, 9 * C + 1, grad + OFF_HEAD_W);
+  k_head_bwd<<<grid, TP, 0, st>>>(gout, ws.head, H, W, ws.y[SI3D_NET_BLOCKS], ws.G, ws.DY, ws.DYb[0]);
+  const int nb = conv_bwd_blocks(B, H, W);
+  for (int k = SI3D_NET_BLOCKS - 1, cur = 0; k >= 0; --k, cur ^= 1) {
+    k_wgrad<C, C, bf16><<<WG_BLOCKS, 32 * WGW, 0, st>>>(ws.x[k], ws.DY, B, H, W, ws.part);
+    k_wgrad_reduce<<<(BLK_SZ + 31) / 32, dim3(32, WR), 0, st>>>(ws.part, WG_BLOCKS, BLK_SZ, grad + OFF_BLK + k * BLK_SZ);
+    k_conv32_bwd<<<nb, 128, 0, st>>>(ws.DYb[cur], ws.wbwd + (size_t)k * 9 * C * C, B, H, W, ws.G, ws.y[k], ws.DY,
+                                     k > 0 ? ws.DYb[cur ^ 1] : nullptr);
   }
-  k_relu_bwd<<<eb, 256, 0, st>>>(G, ws.y[0], ws.DY, nullptr, n);
-  k_wgrad<4, C, float><<<WG_BLOCKS, 256, 0, st>>>(feat, ws.DY, B, H, W, ws.part);
-  k_wgrad_reduce<<<(9 * 4 * C + C + 255) / 256, 256, 0, st>>>(ws.part, WG_BLOCKS, 9 * 4 * C + C, grad);
+  k_wgrad<4, C, float><<<WG_BLOCKS, 32 * WGW, 0, st>>>(feat, ws.DY, B, H, W, ws.part);
+  k_wgrad_reduce<<<(9 * 4 * C + C + 31) / 32, dim3(32, WR), 0, st>>>(ws.part, WG_BLOCKS, 9 * 4 * C + C, grad);
 }
 
 void features(const Dev& d, const int* pix, double* r0, double* part, double* sigma, float* feat, cudaStream_t st) {

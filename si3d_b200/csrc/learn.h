@@ -17,8 +17,8 @@ struct Workspace {
   float *stem = nullptr, *head = nullptr;           // bf16-rounded stem/head weights + biases
   __nv_bfloat16* x[SI3D_NET_BLOCKS + 1] = {};        // activations (layer inputs), channels-last
   float* y[SI3D_NET_BLOCKS + 1] = {};                // pre-activations (training)
-  float *G0 = nullptr, *G1 = nullptr, *DY = nullptr;
-  __nv_bfloat16* DYb = nullptr;
+  float *G = nullptr, *DY = nullptr;
+  __nv_bfloat16* DYb[2] = {nullptr, nullptr};
   float* part = nullptr;                            // weight-gradient partial sums
   bool training = false;
   static size_t bytes(int B, int H, int W, bool training);
