@@ -245,10 +245,13 @@ __global__ void __launch_bounds__(128) k_conv32_bwd(const bf16* __restrict__ Xin
 //                       pixels, N = 32, K = 16, BF16 in, FP32 accumulate) into that row's 32 columns
 //                       of one of two TMEM accumulators, then commits to the accumulator's "full"
 //                       barrier and to the stage's "empty" barrier;
-//   warps 2-5           read the accumulator (each warp its 32 TMEM lanes, i.e. pixels), add bias,
+//   warps 2-17          read the accumulator (each warp its 32 TMEM lanes, i.e. pixels, of its row), add bias,
 //                       ReLU and the residual (from the same stage), store, and release the
 //                       accumulator and the stage.
-// So tile i + 1 loads and tile i multiplies while tile i - 1 is written.  The stage holds
+// So tile i + 1 loads and tile i multiplies while tile i - 1 is written.  Four warps a row of the tile
+// write it: four warps in all could not hide the latency of their own chain (TMEM, shared memory, global
+// memory), and leaving out the loads, the multiplications or the stores changed the time by less than
+// a tenth.  A call at 1002 x 502 pixels 70 -> 38 us, at 32 x 64 x 64 with Y 29 -> 21 us (ncu).  The stage holds
 // [chunk][row][pixel][8 channels]: the A operand of tap (di, dj) for output row r is a K-major
 // no-swizzle matrix starting at row r + 1 + di, pixel 1 + dj (core matrices of 8 pixels x 16 bytes,
 // 128 bytes between pixel groups, one chunk between K halves) - no im2col.  Weights sit as
@@ -265,11 +268,12 @@ constexpr int TC_STAGE = 4 * TC_CHUNK;         // one halo tile
 constexpr int TC_NS = 3;                       // halo tiles in flight
 constexpr int TC_BBYTES = 9 * 4 * C * 16;      // 18,432
 constexpr int TC_OSTRIDE = 80;                 // bytes per pixel of an epilogue warp's staging rows (64 + 16)
-constexpr int TC_OBYTES = 4 * 32 * TC_OSTRIDE; // four epilogue warps x 32 pixels
+constexpr int TC_EW = 4 * TC_R;                // epilogue warps: four a row
+constexpr int TC_OBYTES = TC_EW * 32 * TC_OSTRIDE;   // 32 pixels each
 constexpr int TC_SMEM = TC_NS * TC_STAGE + TC_BBYTES + TC_OBYTES + 1024;   // + alignment of the dynamic base
 constexpr int TC_ACC = TC_R * C;               // TMEM columns of one accumulator (128)
 constexpr int TC_COLS = 2 * TC_ACC;            // two accumulators
-constexpr int TC_THREADS = 192;
+constexpr int TC_THREADS = 64 + 32 * TC_EW;
 constexpr long long TC_WAIT_LIMIT = 1LL << 24; // mbarrier polls before giving up
 static_assert(TC_COLS == 256, "TMEM allocation");
 static_assert(TC_STAGE % 1024 == 0 || TC_CHUNK % 128 == 0, "TMA destinations 128-byte aligned");
@@ -309,7 +313,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv32_tc(const __grid_consta
   extern __shared__ unsigned char smem_raw[];
   __shared__ uint32_t s_tmem;
   __shared__ __align__(8) unsigned long long s_bar[2 * TC_NS + 4];   // full[NS], empty[NS], tfull[2], tempty[2]
-  __shared__ float s_bias[C];
+  __shared__ __align__(16) float s_bias[C];
   __shared__ volatile int s_fail;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const uint32_t rawBase = (uint32_t)__cvta_generic_to_shared(smem_raw);
@@ -333,11 +337,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv32_tc(const __grid_consta
     s_fail = 0;
     for (int st = 0; st < TC_NS; ++st) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" :: "r"(full(st)) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 5;\n" :: "r"(empty(st)) : "memory");   // commit + 4 warps
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n"
+                   :: "r"(empty(st)), "r"(1 + TC_EW) : "memory");   // commit + the epilogue's warps
     }
     for (int a = 0; a < 2; ++a) {
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;\n" :: "r"(tfull(a)) : "memory");
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;\n" :: "r"(tempty(a)) : "memory");
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" :: "r"(tempty(a)), "r"(TC_EW) : "memory");
     }
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
     asm volatile("prefetch.tensormap [%0];\n" :: "l"(reinterpret_cast<uint64_t>(&xmap)) : "memory");
@@ -428,8 +433,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv32_tc(const __grid_consta
       if (issued > 0) tc_wait(tfull((issued - 1) & 1), (uint32_t)(((issued - 1) / 2) & 1), &s_fail);
     }
   } else {
-    // ---------------------------------------------------------------- epilogue (warps 2-5)
-    const int q = warp & 3;              // TMEM lanes 32 q .. 32 q + 31 = pixels of this warp
+    // ---------------------------------------------------------------- epilogue (warps 2-17)
+    const int q = warp & 3, r = (warp - 2) >> 2;   // TMEM lanes 32 q .. 32 q + 31 = pixels of this warp; its row
     const int px = q * 32 + lane;
     // staging rows of this warp's output: the stores to global memory go out as contiguous runs
     unsigned char* const sO = sB + TC_BBYTES + (warp - 2) * 32 * TC_OSTRIDE;
@@ -449,29 +454,64 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv32_tc(const __grid_consta
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;   // the TMEM reads below are warp-collective
       __syncwarp();
       if (ok) asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-      const int gj = j0 + px;
-      for (int r = 0; r < TC_R; ++r) {
-        uint32_t v[C];
-        if (ok) {
-          const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * TC_ACC + r * C);
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-              "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
-              : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-                "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-                "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-              : "r"(taddr) : "memory");
-          asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
-        } else {
+      const int gi = i0 + r;
+      const bool row = gi < H;   // warp-uniform: otherwise the whole row is outside the image
+      uint32_t v[C];
+      if (ok) {
+        const uint32_t taddr = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * TC_ACC + r * C);
+        asm volatile(
+            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
+            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];\n"
+            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+              "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+              "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+            : "r"(taddr) : "memory");
+        asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory");
+      } else {
 #pragma unroll
-          for (int k = 0; k < C; ++k) v[k] = 0u;
+        for (int k = 0; k < C; ++k) v[k] = 0u;
+      }
+      // the stage's values of this pixel; the accumulator and (after these) the stage are given back below
+      const unsigned char* xc = sA + st * TC_STAGE + (r + 1) * TC_ROWB + (px + 1) * 16;
+      const size_t p0 = ((size_t)b * H + gi) * W + (j0 + q * 32);
+      if (row) {
+        float y[C];
+#pragma unroll
+        for (int c4 = 0; c4 < C / 4; ++c4) {
+          const float4 bi = *reinterpret_cast<const float4*>(&s_bias[4 * c4]);
+          y[4 * c4] = __uint_as_float(v[4 * c4]) + bi.x;
+          y[4 * c4 + 1] = __uint_as_float(v[4 * c4 + 1]) + bi.y;
+          y[4 * c4 + 2] = __uint_as_float(v[4 * c4 + 2]) + bi.z;
+          y[4 * c4 + 3] = __uint_as_float(v[4 * c4 + 3]) + bi.w;
         }
-        const int gi = i0 + r;
-        if (gi >= H) continue;   // warp-uniform: the whole row is outside the image
-        const bool inw = gj < W;
-        const size_t p = ((size_t)b * H + gi) * W + gj;
-        const unsigned char* xc = sA + st * TC_STAGE + (r + 1) * TC_ROWB + (px + 1) * 16;
+        if (!ok) {
+#pragma unroll
+          for (int k = 0; k < C; ++k) y[k] = __int_as_float(0x7fc00000);
+        }
+        // Through the staging rows a warp writes 16 bytes a lane: run k, lane l: pixel 8 k + l / 4 and the
+        // l % 4-th 16 bytes of the 64 that were staged for it (X: its 32 channels, Y: half of them)
+        auto flush = [&](unsigned char* out, int stride) {
+          __syncwarp();
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const int pl = k * 8 + (lane >> 2), cc = lane & 3;
+            if (j0 + q * 32 + pl < W)
+              *reinterpret_cast<uint4*>(out + (p0 + pl) * (size_t)stride + cc * 16) =
+                  *reinterpret_cast<const uint4*>(sO + pl * TC_OSTRIDE + cc * 16);
+          }
+          __syncwarp();
+        };
+        if (Y) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+              *reinterpret_cast<float4*>(sO + lane * TC_OSTRIDE + k * 16) =
+                  make_float4(y[h * 16 + 4 * k], y[h * 16 + 4 * k + 1], y[h * 16 + 4 * k + 2], y[h * 16 + 4 * k + 3]);
+            flush(reinterpret_cast<unsigned char*>(Y) + h * 64, C * (int)sizeof(float));
+          }
+        }
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const uint4 xin = ok ? *reinterpret_cast<const uint4*>(xc + c * TC_CHUNK) : make_uint4(0u, 0u, 0u, 0u);
@@ -481,27 +521,13 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv32_tc(const __grid_consta
 #pragma unroll
           for (int e = 0; e < 4; ++e) {
             const int co = c * 8 + 2 * e;
-            float y0 = __uint_as_float(v[co]) + s_bias[co], y1 = __uint_as_float(v[co + 1]) + s_bias[co + 1];
-            if (!ok) { y0 = __int_as_float(0x7fc00000); y1 = y0; }
-            if (Y && inw) *reinterpret_cast<float2*>(Y + p * C + co) = make_float2(y0, y1);
             const float2 xf = __bfloat1622float2(x2[e]);
-            const __nv_bfloat162 ob = __floats2bfloat162_rn(xf.x + fmaxf(y0, 0.f), xf.y + fmaxf(y1, 0.f));
-            o32[e] = *reinterpret_cast<const uint32_t*>(&ob);
+            const __nv_bfloat162 ob = __floats2bfloat162_rn(xf.x + fmaxf(y[co], 0.f), xf.y + fmaxf(y[co + 1], 0.f));
+            o32[e] = ok ? *reinterpret_cast<const uint32_t*>(&ob) : 0x7fc07fc0u;   // (ReLU makes 0 of a NaN)
           }
           *reinterpret_cast<uint4*>(sO + lane * TC_OSTRIDE + c * 16) = o;
         }
-        // the warp's 32 pixels are 2 KB in a row of the output: written as four runs of 512 bytes,
-        // 16 bytes a lane (run k, lane l: pixel 8 k + l / 4, channels 8 (l % 4) ...)
-        __syncwarp();
-        const size_t p0 = ((size_t)b * H + gi) * W + (j0 + q * 32);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          const int byte = k * 512 + lane * 16, pl = byte >> 6, cc = (byte >> 4) & 3;
-          if (j0 + q * 32 + pl < W)
-            *reinterpret_cast<uint4*>(&Xout[(p0 + pl) * C + cc * 8]) =
-                *reinterpret_cast<const uint4*>(sO + pl * TC_OSTRIDE + cc * 16);
-        }
-        __syncwarp();
+        flush(reinterpret_cast<unsigned char*>(Xout), C * (int)sizeof(bf16));
       }
       // this warp is done with the accumulator and the stage
       asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
