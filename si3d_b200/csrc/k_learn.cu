@@ -42,6 +42,20 @@ constexpr int WG_BLOCKS = 296;                 // weight-gradient partial sums (
 
 __device__ __forceinline__ float bfr(float x) { return __bfloat162float(__float2bfloat16_rn(x)); }
 
+// A tile of 32-channel pixels with its frame to shared memory (XS bf16 a pixel), zero outside the
+// image, by asynchronous 16-byte copies: all in flight at once, without a register.  The caller waits.
+template <int ROWS, int COLS, int NT>
+__device__ __forceinline__ void stage_tile(bf16* sX, const bf16* __restrict__ X, int b, int i0, int j0, int H, int W) {
+  for (int r = threadIdx.x; r < ROWS * COLS * 4; r += NT) {
+    const int pix = r >> 2, part = r & 3;
+    const int gi = i0 + pix / COLS - 1, gj = j0 + pix % COLS - 1;
+    const bool in = gi >= 0 && gi < H && gj >= 0 && gj < W;
+    const bf16* src = in ? X + (((size_t)b * H + gi) * W + gj) * C + part * 8 : X;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n"
+                 :: "r"((uint32_t)__cvta_generic_to_shared(&sX[pix * XS + part * 8])), "l"(src), "r"(in ? 16 : 0) : "memory");
+  }
+}
+
 // ------------------------------------------------------------------ weights
 // Block weights to the tensor-core layout [tap][n][k] (bf16): forward n = cout, k = cin;
 // data gradient n = cin, k = cout with the tap mirrored.  Stem/head weights rounded to bf16 values.
@@ -63,74 +77,60 @@ __global__ void k_prep(const float* __restrict__ prm, bf16* __restrict__ wfwd, b
 }
 
 // ------------------------------------------------------------------ stem: 4 -> 32, FP32 cores
-// A block takes 8 rows x 32 pixels; thread (ti, tj) computes pixels tj and tj + 16 of row ti, so each
-// weight it reads from shared memory serves two pixels, and a pixel's four input channels are one
-// 16-byte read.  Per output channel the products are accumulated in the order tap, input channel,
-// with the inputs rounded to BF16 first.
+// A block takes 8 rows x 32 pixels, a warp a row, a lane an output channel with its 36 weights in
+// registers.  The warp walks the row with the 3 x 3 window of the input (four channels each, the same for
+// all lanes) in registers, so a pixel costs three 16-byte broadcasts for 36 FMA, and a pixel's 32
+// channels are stored side by side.  Per output channel the products are accumulated in the order tap,
+// input channel, with the inputs rounded to BF16 first.  Weights from shared memory, a thread all channels
+// of two pixels: 80 us at 1002 x 502 pixels; this: 42 (of which 24 are instruction issue; two pixels'
+// chains interleaved 52, three blocks an SM 43, persistent blocks with the next tile fetched ahead 45).
 constexpr int ST_W = 2 * TW;                   // pixels per row of a stem tile
 constexpr int ST_WT = ST_W + 2;                // with halo
-__global__ void __launch_bounds__(TP) k_stem(const float* __restrict__ feat, const float* __restrict__ w, int H, int W,
-                                             bf16* __restrict__ X, float* __restrict__ Y) {
+__global__ void __launch_bounds__(32 * TH) k_stem(const float* __restrict__ feat, const float* __restrict__ w, int H, int W,
+                                                  bf16* __restrict__ X, float* __restrict__ Y) {
   __shared__ __align__(16) float sF[HT * ST_WT * 4];
-  __shared__ __align__(16) float sW[9 * 4 * C + C];
   const int b = blockIdx.z, i0 = blockIdx.y * TH, j0 = blockIdx.x * ST_W;
-  for (int r = threadIdx.x; r < 9 * 4 * C + C; r += TP) sW[r] = w[r];
-  for (int r = threadIdx.x; r < HT * ST_WT; r += TP) {
+  const int co = threadIdx.x & 31, ti = threadIdx.x >> 5;
+  float wr[36];
+#pragma unroll
+  for (int t = 0; t < 36; ++t) wr[t] = w[t * C + co];
+  const float bias = w[36 * C + co];
+  for (int r = threadIdx.x; r < HT * ST_WT; r += 32 * TH) {
     const int gi = i0 + r / ST_WT - 1, gj = j0 + r % ST_WT - 1;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (gi >= 0 && gi < H && gj >= 0 && gj < W) v = *reinterpret_cast<const float4*>(feat + (((size_t)b * H + gi) * W + gj) * 4);
     *reinterpret_cast<float4*>(&sF[r * 4]) = make_float4(bfr(v.x), bfr(v.y), bfr(v.z), bfr(v.w));
   }
   __syncthreads();
-  const int ti = threadIdx.x / TW, tj = threadIdx.x % TW;
-  float acc[2][C];
-#pragma unroll
-  for (int h = 0; h < 2; ++h)
-#pragma unroll
-    for (int co = 0; co < C; ++co) acc[h][co] = 0.f;
-  for (int t = 0; t < 9; ++t) {
-    const int pi = ti + t / 3, pj = tj + t % 3;   // halo coordinates of the tap's input
-    const float4 va = *reinterpret_cast<const float4*>(&sF[(pi * ST_WT + pj) * 4]);
-    const float4 vb = *reinterpret_cast<const float4*>(&sF[(pi * ST_WT + pj + TW) * 4]);
-    const float xa[4] = {va.x, va.y, va.z, va.w}, xb[4] = {vb.x, vb.y, vb.z, vb.w};
-#pragma unroll
-    for (int ci = 0; ci < 4; ++ci) {
-      const float4* w4 = reinterpret_cast<const float4*>(&sW[(t * 4 + ci) * C]);
-#pragma unroll
-      for (int q = 0; q < C / 4; ++q) {
-        const float4 wq = w4[q];
-        acc[0][4 * q + 0] = __fmaf_rn(xa[ci], wq.x, acc[0][4 * q + 0]);
-        acc[0][4 * q + 1] = __fmaf_rn(xa[ci], wq.y, acc[0][4 * q + 1]);
-        acc[0][4 * q + 2] = __fmaf_rn(xa[ci], wq.z, acc[0][4 * q + 2]);
-        acc[0][4 * q + 3] = __fmaf_rn(xa[ci], wq.w, acc[0][4 * q + 3]);
-        acc[1][4 * q + 0] = __fmaf_rn(xb[ci], wq.x, acc[1][4 * q + 0]);
-        acc[1][4 * q + 1] = __fmaf_rn(xb[ci], wq.y, acc[1][4 * q + 1]);
-        acc[1][4 * q + 2] = __fmaf_rn(xb[ci], wq.z, acc[1][4 * q + 2]);
-        acc[1][4 * q + 3] = __fmaf_rn(xb[ci], wq.w, acc[1][4 * q + 3]);
-      }
-    }
-  }
   const int gi = i0 + ti;
+  if (gi >= H) return;
+  const size_t p0 = ((size_t)b * H + gi) * W + j0;
+  const int n = min(ST_W, W - j0);
+  float4 x[3][3];   // rows, columns of the window
+  auto column = [&](int c, int tj) {
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
-    const int gj = j0 + tj + h * TW;
-    if (gi >= H || gj >= W) continue;
-    const size_t p = ((size_t)b * H + gi) * W + gj;
-    // the pixel's 32 channels as four 16-byte stores
+    for (int i = 0; i < 3; ++i) x[i][c] = *reinterpret_cast<const float4*>(&sF[((ti + i) * ST_WT + tj) * 4]);
+  };
+  column(0, 0);
+  column(1, 1);
+#pragma unroll 4
+  for (int tj = 0; tj < n; ++tj) {
+    column(2, tj + 2);
+    float acc = 0.f;
 #pragma unroll
-    for (int c4 = 0; c4 < C / 8; ++c4) {
-      uint4 o;
-      uint32_t* o32 = reinterpret_cast<uint32_t*>(&o);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const int co = c4 * 8 + 2 * e;
-        const float y0 = acc[h][co] + sW[9 * 4 * C + co], y1 = acc[h][co + 1] + sW[9 * 4 * C + co + 1];
-        if (Y) *reinterpret_cast<float2*>(Y + p * C + co) = make_float2(y0, y1);
-        const __nv_bfloat162 ob = __floats2bfloat162_rn(fmaxf(y0, 0.f), fmaxf(y1, 0.f));
-        o32[e] = *reinterpret_cast<const uint32_t*>(&ob);
-      }
-      *reinterpret_cast<uint4*>(X + p * C + c4 * 8) = o;
+    for (int t = 0; t < 9; ++t) {
+      const float4 v = x[t / 3][t % 3];
+      acc = __fmaf_rn(v.x, wr[4 * t], acc);
+      acc = __fmaf_rn(v.y, wr[4 * t + 1], acc);
+      acc = __fmaf_rn(v.z, wr[4 * t + 2], acc);
+      acc = __fmaf_rn(v.w, wr[4 * t + 3], acc);
     }
+    const float y = acc + bias;
+    const size_t o = (p0 + tj) * C + co;
+    if (Y) Y[o] = y;
+    X[o] = __float2bfloat16_rn(fmaxf(y, 0.f));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) { x[i][0] = x[i][1]; x[i][1] = x[i][2]; }
   }
 }
 
@@ -147,13 +147,14 @@ __device__ __forceinline__ void mma_bf16(float* c, uint32_t a0, uint32_t a1, uin
 // Behind a layer's G (the gradient of its input x_k): DY = G * (y_k > 0), the gradient at the ReLU of
 // the layer below, in FP32 for the weight gradient and (unless it is the stem's) in BF16 for the
 // tensor-core data gradient.  Written by the kernel that makes G, which spares a pass over G a layer
-// (32 x 64 x 64 pixels: five passes of 19.5 us; the data gradient takes 32.6 instead of 25.5 us).
+// (32 x 64 x 64 pixels: five passes of 19.5 us against 7 us more in the data gradient).
 __device__ __forceinline__ float relu_grad(float g, float y) { return y > 0.f ? g : 0.f; }
 
 // Data gradient of a 32 -> 32 layer: G[p][n] += sum_{tap, k} in[p + off(tap)][k] * Wk[tap][n][k], in place
 // (a thread reads and writes the same elements), and for the layer below DY and (not for the stem) DYb
 // from its y.  Persistent blocks: the weights go to shared memory once per block, which then loops over
-// 8 x 16 pixel tiles (tile = blockIdx.x, blockIdx.x + gridDim.x, ...).
+// 8 x 16 pixel tiles (tile = blockIdx.x, blockIdx.x + gridDim.x, ...).  Tiles by asynchronous copies and a
+// row's G and Y loaded together: 32.6 -> 26.4 us at 32 x 64 x 64 pixels (84 MB: 13 us at memory's rate).
 __global__ void __launch_bounds__(128) k_conv32_bwd(const bf16* __restrict__ Xin, const bf16* __restrict__ Wk, int B,
                                                     int H, int W, float* __restrict__ G, const float* __restrict__ Y,
                                                     float* __restrict__ DY, bf16* __restrict__ DYb) {
@@ -168,14 +169,8 @@ __global__ void __launch_bounds__(128) k_conv32_bwd(const bf16* __restrict__ Xin
     const int b = tile / (nti * ntj), rem = tile - b * (nti * ntj);
     const int i0 = (rem / ntj) * TH, j0 = (rem % ntj) * TW;
     __syncthreads();   // the previous tile's readers of sX are done
-    for (int r = threadIdx.x; r < HT * WT * 4; r += 128) {
-      const int pix = r >> 2, part = r & 3;
-      const int gi = i0 + pix / WT - 1, gj = j0 + pix % WT - 1;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (gi >= 0 && gi < H && gj >= 0 && gj < W)
-        v = *reinterpret_cast<const uint4*>(&Xin[(((size_t)b * H + gi) * W + gj) * C + part * 8]);
-      *reinterpret_cast<uint4*>(&sX[pix * XS + part * 8]) = v;
-    }
+    stage_tile<HT, WT, 128>(sX, Xin, b, i0, j0, H, W);
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
     float acc[2][4][4];
@@ -212,18 +207,30 @@ __global__ void __launch_bounds__(128) k_conv32_bwd(const bf16* __restrict__ Xin
     }
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int ty = warp * 2 + r, gi = i0 + ty;
+      const int gi = i0 + warp * 2 + r;
+      if (gi >= H) continue;
+      const size_t o0 = (((size_t)b * H + gi) * W + j0) * C + 2 * q;
+      float2 gin[2][4], y[2][4];   // the row's values, all loads in flight at once
 #pragma unroll
       for (int half = 0; half < 2; ++half) {
-        const int tj = g + 8 * half, gj = j0 + tj;
-        if (gi >= H || gj >= W) continue;
-        const size_t p = ((size_t)b * H + gi) * W + gj;
+        const int tj = g + 8 * half;
+        if (j0 + tj < W) {
+#pragma unroll
+          for (int nt = 0; nt < 4; ++nt) {
+            gin[half][nt] = *reinterpret_cast<const float2*>(G + o0 + tj * C + nt * 8);
+            y[half][nt] = *reinterpret_cast<const float2*>(Y + o0 + tj * C + nt * 8);
+          }
+        }
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        const int tj = g + 8 * half;
+        if (j0 + tj >= W) continue;
 #pragma unroll
         for (int nt = 0; nt < 4; ++nt) {
-          const size_t o = p * C + nt * 8 + 2 * q;
-          const float2 gi2 = *reinterpret_cast<const float2*>(G + o), y = *reinterpret_cast<const float2*>(Y + o);
-          const float2 go = make_float2(gi2.x + acc[r][nt][2 * half], gi2.y + acc[r][nt][2 * half + 1]);
-          const float2 d = make_float2(relu_grad(go.x, y.x), relu_grad(go.y, y.y));
+          const size_t o = o0 + tj * C + nt * 8;
+          const float2 go = make_float2(gin[half][nt].x + acc[r][nt][2 * half], gin[half][nt].y + acc[r][nt][2 * half + 1]);
+          const float2 d = make_float2(relu_grad(go.x, y[half][nt].x), relu_grad(go.y, y[half][nt].y));
           *reinterpret_cast<float2*>(DY + o) = d;
           if (DYb) {
             *reinterpret_cast<float2*>(G + o) = go;
@@ -548,42 +555,57 @@ __global__ void __launch_bounds__(TC_THREADS, 1) k_conv32_tc(const __grid_consta
 }
 
 // ------------------------------------------------------------------ head: 32 -> 1, FP32 cores
-__global__ void __launch_bounds__(TP) k_head(const bf16* __restrict__ X, const float* __restrict__ w, int H, int W,
-                                             float* __restrict__ out) {
-  __shared__ __align__(16) bf16 sX[HT * WT * XS];
+// A thread computes four pixels of a column (tile: 8 rows x 32 pixels): a value of X read from shared
+// memory and widened serves three rows of taps, a weight four pixels.  The products of an output are
+// accumulated in the order tap column, eight channels, tap row.  A pixel a thread 31 us at 1002 x 502
+// pixels; this with plain loads for the tile 29, with asynchronous copies 22.
+constexpr int HD_R = 4;                        // pixels of a thread
+constexpr int HD_T = TH / HD_R * ST_W;         // threads
+__global__ void __launch_bounds__(HD_T) k_head(const bf16* __restrict__ X, const float* __restrict__ w, int H, int W,
+                                               float* __restrict__ out) {
+  __shared__ __align__(16) bf16 sX[HT * ST_WT * XS];
   __shared__ __align__(16) float sW[9 * C + 1];
-  const int b = blockIdx.z, i0 = blockIdx.y * TH, j0 = blockIdx.x * TW;
-  for (int r = threadIdx.x; r < 9 * C + 1; r += TP) sW[r] = w[r];
-  for (int r = threadIdx.x; r < HT * WT * 4; r += TP) {
-    const int pix = r >> 2, part = r & 3;
-    const int gi = i0 + pix / WT - 1, gj = j0 + pix % WT - 1;
-    uint4 v = make_uint4(0u, 0u, 0u, 0u);
-    if (gi >= 0 && gi < H && gj >= 0 && gj < W)
-      v = *reinterpret_cast<const uint4*>(&X[(((size_t)b * H + gi) * W + gj) * C + part * 8]);
-    *reinterpret_cast<uint4*>(&sX[pix * XS + part * 8]) = v;
-  }
+  const int b = blockIdx.z, i0 = blockIdx.y * TH, j0 = blockIdx.x * ST_W;
+  for (int r = threadIdx.x; r < 9 * C + 1; r += HD_T) sW[r] = w[r];
+  stage_tile<HT, ST_WT, HD_T>(sX, X, b, i0, j0, H, W);
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
   __syncthreads();
-  const int ti = threadIdx.x / TW, tj = threadIdx.x % TW;
-  const int gi = i0 + ti, gj = j0 + tj;
-  if (gi >= H || gj >= W) return;
-  float acc = 0.f;
-  for (int t = 0; t < 9; ++t) {
-    const uint4* xp = reinterpret_cast<const uint4*>(&sX[((ti + t / 3) * WT + tj + t % 3) * XS]);
-    const float4* w4 = reinterpret_cast<const float4*>(&sW[t * C]);
+  const int t0 = threadIdx.x / ST_W * HD_R, tj = threadIdx.x % ST_W, gj = j0 + tj;
+  if (gj >= W) return;
+  float acc[HD_R];
+#pragma unroll
+  for (int i = 0; i < HD_R; ++i) acc[i] = 0.f;
+  for (int dj = 0; dj < 3; ++dj) {
 #pragma unroll
     for (int q = 0; q < C / 8; ++q) {
-      const uint4 xv = xp[q];
-      const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&xv);
-      const float4 wa = w4[2 * q], wb = w4[2 * q + 1];
-      const float2 f0 = __bfloat1622float2(x2[0]), f1 = __bfloat1622float2(x2[1]);
-      const float2 f2 = __bfloat1622float2(x2[2]), f3 = __bfloat1622float2(x2[3]);
-      acc = __fmaf_rn(f0.x, wa.x, acc); acc = __fmaf_rn(f0.y, wa.y, acc);
-      acc = __fmaf_rn(f1.x, wa.z, acc); acc = __fmaf_rn(f1.y, wa.w, acc);
-      acc = __fmaf_rn(f2.x, wb.x, acc); acc = __fmaf_rn(f2.y, wb.y, acc);
-      acc = __fmaf_rn(f3.x, wb.z, acc); acc = __fmaf_rn(f3.y, wb.w, acc);
+      float wv[3][8];
+#pragma unroll
+      for (int di = 0; di < 3; ++di) {
+        const float4* w4 = reinterpret_cast<const float4*>(&sW[(di * 3 + dj) * C + 8 * q]);
+        const float4 a = w4[0], c = w4[1];
+        wv[di][0] = a.x; wv[di][1] = a.y; wv[di][2] = a.z; wv[di][3] = a.w;
+        wv[di][4] = c.x; wv[di][5] = c.y; wv[di][6] = c.z; wv[di][7] = c.w;
+      }
+#pragma unroll
+      for (int i = 0; i < HD_R + 2; ++i) {   // halo rows: row i is tap row di of pixel i - di
+        const uint4 xv = *reinterpret_cast<const uint4*>(&sX[((t0 + i) * ST_WT + tj + dj) * XS + 8 * q]);
+        const __nv_bfloat162* x2 = reinterpret_cast<const __nv_bfloat162*>(&xv);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __bfloat1622float2(x2[e]);
+#pragma unroll
+          for (int di = 0; di < 3; ++di)
+            if (i - di >= 0 && i - di < HD_R) {
+              acc[i - di] = __fmaf_rn(f.x, wv[di][2 * e], acc[i - di]);
+              acc[i - di] = __fmaf_rn(f.y, wv[di][2 * e + 1], acc[i - di]);
+            }
+        }
+      }
     }
   }
-  out[((size_t)b * H + gi) * W + gj] = acc + sW[9 * C];
+#pragma unroll
+  for (int i = 0; i < HD_R; ++i)
+    if (i0 + t0 + i < H) out[((size_t)b * H + i0 + t0 + i) * W + gj] = acc[i] + sW[9 * C];
 }
 
 // ------------------------------------------------------------------ backward pieces
@@ -628,46 +650,170 @@ __global__ void __launch_bounds__(TP) k_head_bwd(const float* __restrict__ gout,
 }
 
 // Weight gradient partials: part[blk][(tap * CIN + ci) * COUT + co] = sum over the block's tiles of
-// X[p + off(tap)][ci] * DY[p][co], and part[blk][9 * CIN * COUT + co] = sum DY[p][co].  FP32 on the FP32
-// cores (DY is held in FP32).  A tile's X (one pixel of frame) and DY are staged in shared memory, and a
-// thread walks the tile's pixels row by row with the 3 x 3 window of X in registers, so a pixel costs
-// three loads of X whatever the number of taps.  What a lane and a warp own depends on the layer:
-//   32 -> 32  lane = ci, warp = four co: 9 x 4 sums a thread, all pixels (40 instructions for 36 FMA)
-//    4 -> 32  lane = co, four ci a thread (one 16-byte load of X): 36 sums, the warps share the rows
-//   32 -> 1   lane = ci: 9 sums, the warps share the rows
-// The warps that share rows add their sums at the end in a fixed order.  The next
+// X[p + off(tap)][ci] * DY[p][co], and part[blk][9 * CIN * COUT + co] = sum DY[p][co].
+constexpr int GH = 4, GP = GH * TW;        // tiles: 4 x 16 pixels
+constexpr int GHP = (GH + 2) * WT;         // with frame
+
+// 32 -> 32.  X is BF16 and DY FP32.  DY is cut into three BF16 terms of eight bits each, whose sum is DY
+// exactly, so the tensor cores form the same products as FP32 multiply-adds, X * DY, and sum them in
+// FP32.  A warp has one tap: M = 32 ci, N = 32 co, K = 16 pixels of a row, A and B by transposed
+// ldmatrix from pixel-major tiles (80 bytes a pixel: no bank conflicts).  The next tile's X (cp.async)
+// and DY (registers) are under way behind the multiplications.  The tensor core cuts where an FP32 add
+// rounds, so its sums are kept short: 16 pixels of a row, three products, then an FP32 add to the
+// thread's sums.  Error against 64 bits (relative, L2 over the gradient; six cases of 128 to 131,072
+// pixels): 0.7e-7 to 1.7e-7, of FP32 multiply-adds 1.1e-7 to 3.9e-7; with one chain a tile or a block it
+// would be up to 3 times that of FP32.  32 x 64 x 64 pixels, per call: FP32 cores, one load a multiply-add
+// 200 us; FP32 cores, 9 x 4 sums a thread 66 (9 x 8: 67, packed pairs: 65; bound by the FP32 pipes); this: 32.
+// An infinite DY gives infinities (its lower terms are zero), except against an infinite X: NaN.
+constexpr int GT = 9 * 32;                 // threads: a warp a tap
+__device__ __forceinline__ void ldsm4t(uint32_t* r, const bf16* p) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((uint32_t)__cvta_generic_to_shared(p)) : "memory");
+}
+__device__ __forceinline__ uint32_t top_halves(float a, float b) {   // two FP32 cut to BF16, a in the low half
+  return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
+}
+__device__ __forceinline__ float cut(float a) { return __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
+__device__ __forceinline__ float rest(float a) { return isinf(a) ? 0.f : a - cut(a); }   // exact
+
+__global__ void __launch_bounds__(GT, 2) k_wgrad32(const bf16* __restrict__ X, const float* __restrict__ DY, int B, int H,
+                                                   int W, float* __restrict__ part) {
+  __shared__ __align__(16) bf16 sX[2][GHP * XS];
+  __shared__ __align__(16) bf16 sD[3][GP * XS];
+  constexpr int ND = (GP * C / 4 + GT - 1) / GT;   // float4 of DY a thread stages
+  const int ln = threadIdx.x & 31, tap = threadIdx.x >> 5;
+  const int nj = (W + TW - 1) / TW, ni = (H + GH - 1) / GH, ntiles = B * ni * nj;
+  const int c4 = threadIdx.x % (C / 4) * 4;        // the channels it stages (GT is a multiple of 8)
+  float acc[2][4][4];                              // [ci / 16][co / 8][fragment]
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), rd[ND];
+  auto fetch = [&](int tile, int buf) {
+    const int b = tile / (ni * nj), rem = tile - b * (ni * nj), i0 = rem / nj * GH, j0 = rem % nj * TW;
+    stage_tile<GH + 2, WT, GT>(sX[buf], X, b, i0, j0, H, W);
+#pragma unroll
+    for (int k = 0; k < ND; ++k) {
+      const int pix = (threadIdx.x + k * GT) / (C / 4), gi = i0 + pix / TW, gj = j0 + pix % TW;
+      rd[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (pix < GP && gi < H && gj < W)
+        rd[k] = *reinterpret_cast<const float4*>(DY + (((size_t)b * H + gi) * W + gj) * C + c4);
+    }
+  };
+  int buf = 0;
+  if ((int)blockIdx.x < ntiles) fetch(blockIdx.x, 0);
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+    __syncthreads();   // the previous tile's readers are done
+#pragma unroll
+    for (int k = 0; k < ND; ++k) {
+      const int pix = (threadIdx.x + k * GT) / (C / 4);
+      float4 d = rd[k];
+      sum.x = sum.x + d.x; sum.y = sum.y + d.y; sum.z = sum.z + d.z; sum.w = sum.w + d.w;
+      if (pix < GP) {
+#pragma unroll
+        for (int s = 0; s < 3; ++s) {
+          *reinterpret_cast<uint2*>(&sD[s][pix * XS + c4]) = make_uint2(top_halves(d.x, d.y), top_halves(d.z, d.w));
+          d = make_float4(rest(d.x), rest(d.y), rest(d.z), rest(d.w));
+        }
+      }
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x, buf ^ 1);
+    const bf16* xa = &sX[buf][((tap / 3) * WT + tap % 3 + (ln & 7) + (ln >> 4) * 8) * XS + ((ln >> 3) & 1) * 8];
+    const int ob = ((ln & 7) + ((ln >> 3) & 1) * 8) * XS + (ln >> 4) * 8;
+#pragma unroll
+    for (int ti = 0; ti < GH; ++ti) {
+      uint32_t a[2][4];
+      ldsm4t(a[0], xa + ti * WT * XS);
+      ldsm4t(a[1], xa + ti * WT * XS + 16);
+#pragma unroll
+      for (int n2 = 0; n2 < 2; ++n2) {
+        float r[2][2][4];   // the sums over this row's 16 pixels
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) r[m][0][e] = r[m][1][e] = 0.f;
+#pragma unroll
+        for (int s = 2; s >= 0; --s) {   // the small terms first
+          uint32_t bq[4];
+          ldsm4t(bq, &sD[s][ti * TW * XS + ob + n2 * 16]);
+#pragma unroll
+          for (int m = 0; m < 2; ++m) {
+            mma_bf16(r[m][0], a[m][0], a[m][1], a[m][2], a[m][3], bq[0], bq[1]);
+            mma_bf16(r[m][1], a[m][0], a[m][1], a[m][2], a[m][3], bq[2], bq[3]);
+          }
+        }
+#pragma unroll
+        for (int m = 0; m < 2; ++m)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            acc[m][2 * n2][e] = acc[m][2 * n2][e] + r[m][0][e];
+            acc[m][2 * n2 + 1][e] = acc[m][2 * n2 + 1][e] + r[m][1][e];
+          }
+      }
+    }
+  }
+  float* o = part + (size_t)blockIdx.x * BLK_SZ;
+  const int g = ln >> 2, q = ln & 3;
+#pragma unroll
+  for (int m = 0; m < 2; ++m)
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        *reinterpret_cast<float2*>(&o[(tap * C + m * 16 + g + 8 * h) * C + n * 8 + 2 * q]) =
+            make_float2(acc[m][n][2 * h], acc[m][n][2 * h + 1]);
+  // the bias: the staging threads' sums, in the threads' order
+  __syncthreads();
+  float* sS = reinterpret_cast<float*>(&sD[0][0]);   // [GT / 8][32]
+  static_assert(GT / 8 * 32 * sizeof(float) <= sizeof(sD), "room for the sums");
+  *reinterpret_cast<float4*>(&sS[threadIdx.x / (C / 4) * C + c4]) = sum;
+  __syncthreads();
+  if (threadIdx.x < C) {
+    float v = sS[threadIdx.x];
+    for (int r = 1; r < GT / 8; ++r) v = v + sS[r * C + threadIdx.x];
+    o[9 * C * C + threadIdx.x] = v;
+  }
+}
+
+// The stem's and the head's, FP32: a tile's X and DY are staged in shared memory, and a thread walks
+// pixels with the 3 x 3 window of X in registers, so a pixel costs three loads of X for all taps.
+//    4 -> 32  lane = co, four ci a thread (one 16-byte load of X): 36 sums
+//   32 -> 1   lane = ci: 9 sums
+// A warp takes half a row of a tile; the warps' sums are added at the end in a fixed order.  The next
 // tile's values are fetched into registers behind the tile's arithmetic.  32 x 64 x 64 pixels, per call,
-// with one load of X per multiply-add and no FMA -> this: 200 -> 66, 57 -> 16 and 63 -> 11 us (8 x 16
-// pixel tiles without the fetch ahead: 94, 29, 44).
+// with one load of X per multiply-add and no FMA -> this: 57 -> 16 and 63 -> 11 us (8 x 16 pixel tiles
+// without the fetch ahead: 29, 44).
 constexpr int WGW = 8;                     // warps of a weight-gradient block
-constexpr int GH = 4, GP = GH * TW;        // its tiles: 4 x 16 pixels
-constexpr int GHP = (GH + 2) * WT;         // with halo
 template <int CIN, int COUT, typename XT>
 __global__ void __launch_bounds__(32 * WGW, 2) k_wgrad(const XT* __restrict__ X, const float* __restrict__ DY, int B,
                                                        int H, int W, float* __restrict__ part) {
-  constexpr bool FULL = CIN == 32 && COUT == 32;   // the three shapes of the network
   constexpr bool STEM = CIN == 4 && COUT == 32;
-  static_assert(FULL || STEM || (CIN == 32 && COUT == 1), "layer shape");
+  static_assert(STEM || (CIN == 32 && COUT == 1), "layer shape");
+  static_assert(WGW == 2 * GH, "half a row a warp");
   constexpr int NTH = 32 * WGW;
   constexpr int R = 9 * CIN, NOUT = R * COUT + COUT;
-  constexpr int NQ = FULL || STEM ? 4 : 1;   // FULL: values of DY a window value meets; STEM: channels of a window pixel
-  constexpr int NX = STEM ? 4 : 1, ND = FULL ? 4 : 1;
-  constexpr int XV = CIN == 32 ? 8 : 1, NXL = (GHP * CIN / XV + NTH - 1) / NTH;     // loads of X a thread, values each
-  constexpr int DV = COUT == 32 ? 4 : 1, NDL = (GP * COUT / DV + NTH - 1) / NTH;    // of DY
+  constexpr int NX = STEM ? 4 : 1;           // channels of a window pixel in a thread
+  constexpr int NA = 9 * NX + 1;             // sums of a thread
+  constexpr int XV = STEM ? 1 : 8, NXL = (GHP * CIN / XV + NTH - 1) / NTH;     // loads of X a thread, values each
+  constexpr int DV = STEM ? 4 : 1, NDL = (GP * COUT / DV + NTH - 1) / NTH;     // of DY
   __shared__ __align__(16) float sX[GHP * CIN];
   __shared__ __align__(16) float sD[GP * COUT];
+  __shared__ float sA[WGW][NA * 32];
   const int ln = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int nj = (W + TW - 1) / TW, ni = (H + GH - 1) / GH, ntiles = B * ni * nj;
-  float acc[9][NQ], accb[ND];
+  float acc[9][NX], accb = 0.f;
 #pragma unroll
-  for (int q = 0; q < ND; ++q) accb[q] = 0.f;
+  for (int t = 0; t < 9; ++t)
 #pragma unroll
-  for (int q = 0; q < NQ; ++q)
-#pragma unroll
-    for (int t = 0; t < 9; ++t) acc[t][q] = 0.f;
-  uint4 rx[CIN == 32 ? NXL : 1];
-  float rxf[CIN == 32 ? 1 : NXL];
-  float4 rd[COUT == 32 ? NDL : 1];
+    for (int q = 0; q < NX; ++q) acc[t][q] = 0.f;
+  uint4 rx[STEM ? 1 : NXL];
+  float rxf[STEM ? NXL : 1];
+  float4 rd[STEM ? NDL : 1];
   float rdf = 0.f;
   auto fetch = [&](int tile) {   // a tile's X (zero outside the image) and DY to registers
     const int b = tile / (ni * nj), rem = tile - b * (ni * nj), i0 = rem / nj * GH, j0 = rem % nj * TW;
@@ -677,11 +823,11 @@ __global__ void __launch_bounds__(32 * WGW, 2) k_wgrad(const XT* __restrict__ X,
       const int gi = i0 + pix / WT - 1, gj = j0 + pix % WT - 1;
       const bool in = pix < GHP && gi >= 0 && gi < H && gj >= 0 && gj < W;
       const size_t o = (((size_t)b * H + gi) * W + gj) * CIN + c;
-      if constexpr (CIN == 32) {
+      if constexpr (STEM) {
+        rxf[k] = in ? bfr(X[o]) : 0.f;
+      } else {
         rx[k] = make_uint4(0u, 0u, 0u, 0u);
         if (in) rx[k] = *reinterpret_cast<const uint4*>(X + o);
-      } else {
-        rxf[k] = in ? bfr(X[o]) : 0.f;
       }
     }
 #pragma unroll
@@ -690,7 +836,7 @@ __global__ void __launch_bounds__(32 * WGW, 2) k_wgrad(const XT* __restrict__ X,
       const int gi = i0 + pix / TW, gj = j0 + pix % TW;
       const bool in = pix < GP && gi < H && gj < W;
       const size_t o = (((size_t)b * H + gi) * W + gj) * COUT + c;
-      if constexpr (COUT == 32) {
+      if constexpr (STEM) {
         rd[k] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (in) rd[k] = *reinterpret_cast<const float4*>(DY + o);
       } else {
@@ -705,14 +851,14 @@ __global__ void __launch_bounds__(32 * WGW, 2) k_wgrad(const XT* __restrict__ X,
     for (int k = 0; k < NXL; ++k) {
       const int r = threadIdx.x + k * NTH;
       if (r * XV < GHP * CIN) {
-        if constexpr (CIN == 32) {
+        if constexpr (STEM) {
+          sX[r] = rxf[k];
+        } else {
           const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&rx[k]);
           const float2 a = __bfloat1622float2(h[0]), b = __bfloat1622float2(h[1]);
           const float2 c = __bfloat1622float2(h[2]), d = __bfloat1622float2(h[3]);
           *reinterpret_cast<float4*>(&sX[r * 8]) = make_float4(a.x, a.y, b.x, b.y);
           *reinterpret_cast<float4*>(&sX[r * 8 + 4]) = make_float4(c.x, c.y, d.x, d.y);
-        } else {
-          sX[r] = rxf[k];
         }
       }
     }
@@ -720,85 +866,60 @@ __global__ void __launch_bounds__(32 * WGW, 2) k_wgrad(const XT* __restrict__ X,
     for (int k = 0; k < NDL; ++k) {
       const int r = threadIdx.x + k * NTH;
       if (r * DV < GP * COUT) {
-        if constexpr (COUT == 32) *reinterpret_cast<float4*>(&sD[r * 4]) = rd[k];
+        if constexpr (STEM) *reinterpret_cast<float4*>(&sD[r * 4]) = rd[k];
         else sD[r] = rdf;
       }
     }
     __syncthreads();
     if (tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x);   // lands behind this tile's arithmetic
-    // FULL: every warp walks all rows; the others: half a row a warp
-    constexpr int LEN = FULL ? TW : TW / 2;
-    static_assert(FULL || WGW == 2 * GH, "half a row a warp");
-    for (int u = FULL ? 0 : wp; u < (FULL ? GH : wp + 1); ++u) {
-      const int ti = FULL ? u : u >> 1, t0 = FULL ? 0 : (u & 1) * LEN;
-      float x[3][3][NX];   // the 3 x 3 window of X (STEM: four channels of each)
-      auto column = [&](int c, int tj) {   // window column c from image column tj - 1
+    const int ti = wp >> 1, t0 = (wp & 1) * (TW / 2);
+    float x[3][3][NX];   // the 3 x 3 window of X
+    auto column = [&](int c, int tj) {   // window column c from image column tj - 1
 #pragma unroll
-        for (int i = 0; i < 3; ++i) {
-          const int o = ((ti + i) * WT + tj) * CIN;
-          if constexpr (STEM) {
-            const float4 v = *reinterpret_cast<const float4*>(&sX[o]);
-            x[i][c][0] = v.x; x[i][c][1] = v.y; x[i][c][2] = v.z; x[i][c][3] = v.w;
-          } else {
-            x[i][c][0] = sX[o + ln];
-          }
-        }
-      };
-      column(0, t0);
-      column(1, t0 + 1);
-#pragma unroll 4
-      for (int tj = t0; tj < t0 + LEN; ++tj) {
-        column(2, tj + 2);
-        const float* dp = &sD[(ti * TW + tj) * COUT];
-        float d[ND];
-        if constexpr (FULL) {
-          const float4 v = *reinterpret_cast<const float4*>(dp + 4 * wp);
-          d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
+      for (int i = 0; i < 3; ++i) {
+        const int o = ((ti + i) * WT + tj) * CIN;
+        if constexpr (STEM) {
+          const float4 v = *reinterpret_cast<const float4*>(&sX[o]);
+          x[i][c][0] = v.x; x[i][c][1] = v.y; x[i][c][2] = v.z; x[i][c][3] = v.w;
         } else {
-          d[0] = dp[STEM ? ln : 0];
+          x[i][c][0] = sX[o + ln];
         }
-#pragma unroll
-        for (int q = 0; q < ND; ++q) accb[q] = accb[q] + d[q];
-#pragma unroll
-        for (int t = 0; t < 9; ++t)
-#pragma unroll
-          for (int q = 0; q < NQ; ++q) acc[t][q] = fmaf(x[t / 3][t % 3][STEM ? q : 0], d[FULL ? q : 0], acc[t][q]);
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-          for (int q = 0; q < NX; ++q) { x[i][0][q] = x[i][1][q]; x[i][1][q] = x[i][2][q]; }
       }
+    };
+    column(0, t0);
+    column(1, t0 + 1);
+#pragma unroll 4
+    for (int tj = t0; tj < t0 + TW / 2; ++tj) {
+      column(2, tj + 2);
+      const float d = sD[(ti * TW + tj) * COUT + (STEM ? ln : 0)];
+      accb = accb + d;
+#pragma unroll
+      for (int t = 0; t < 9; ++t)
+#pragma unroll
+        for (int q = 0; q < NX; ++q) acc[t][q] = fmaf(x[t / 3][t % 3][q], d, acc[t][q]);
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int q = 0; q < NX; ++q) { x[i][0][q] = x[i][1][q]; x[i][1][q] = x[i][2][q]; }
     }
   }
   float* o = part + (size_t)blockIdx.x * NOUT;
-  if constexpr (FULL) {
 #pragma unroll
-    for (int t = 0; t < 9; ++t)
-      *reinterpret_cast<float4*>(&o[(t * CIN + ln) * COUT + 4 * wp]) = make_float4(acc[t][0], acc[t][1], acc[t][2], acc[t][3]);
-    if (ln == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; ++q) o[R * COUT + 4 * wp + q] = accb[q];
-    }
-  } else {
-    // the warps' sums of each output, added warp by warp
-    constexpr int NA = 9 * NQ + 1;   // sums of a thread
-    __shared__ float sA[WGW][NA * 32];
-#pragma unroll
-    for (int m = 0; m < NA; ++m) sA[wp][m * 32 + ln] = m < 9 * NQ ? acc[m / NQ % 9][m % NQ] : accb[0];
-    __syncthreads();
-    for (int r = threadIdx.x; r < NA * 32; r += NTH) {
-      const int m = r >> 5, l = r & 31;
-      float v = sA[0][r];
-      for (int w = 1; w < WGW; ++w) v = v + sA[w][r];
-      if (m < 9 * NQ) o[STEM ? m * COUT + l : m * CIN + l] = v;   // m = tap (x 4 + ci)
-      else if (STEM || l == 0) o[R * COUT + l] = v;
-    }
+  for (int m = 0; m < NA; ++m) sA[wp][m * 32 + ln] = m < 9 * NX ? acc[m / NX % 9][m % NX] : accb;
+  __syncthreads();
+  for (int r = threadIdx.x; r < NA * 32; r += NTH) {
+    const int m = r >> 5, l = r & 31;
+    float v = sA[0][r];
+    for (int w = 1; w < WGW; ++w) v = v + sA[w][r];
+    if (m < 9 * NX) o[STEM ? m * COUT + l : m * CIN + l] = v;   // m = tap (x 4 + ci)
+    else if (STEM || l == 0) o[R * COUT + l] = v;
   }
 }
 
 // grad[off + o] = sum_blk part[blk][o] (fixed order: WR threads of an output each take every WR-th block,
 // then their sums in order); the weight part [9][CIN][COUT] first, then the COUT bias entries.  One
-// thread per output left three SMs in four idle (21 us for the 9248 outputs of a block, 8.6 so).
+// thread per output left three SMs in four idle (21 us for the 9248 outputs of a block, 8.5 so; 32 threads an output 7.7,
+// but a larger rounding error).
 constexpr int WR = 8;
 __global__ void __launch_bounds__(32 * WR) k_wgrad_reduce(const float* __restrict__ part, int nblk, int nout,
                                                           float* __restrict__ grad) {
@@ -806,7 +927,7 @@ __global__ void __launch_bounds__(32 * WR) k_wgrad_reduce(const float* __restric
   const int o = blockIdx.x * 32 + threadIdx.x;
   float s = 0.f;
   if (o < nout) {
-#pragma unroll 4
+#pragma unroll 10
     for (int b = threadIdx.y; b < nblk; b += WR) s = s + part[(size_t)b * nout + o];
   }
   sh[threadIdx.y][threadIdx.x] = s;
@@ -838,10 +959,15 @@ __global__ void k_loss_part(const float* __restrict__ out, const float* __restri
   if (threadIdx.x == 0) { part[2 * blockIdx.x] = s1[0]; part[2 * blockIdx.x + 1] = s2[0]; }
 }
 
+constexpr int LOSS_BLOCKS = 148;   // blocks of k_loss_part
 __global__ void k_loss_final(const float* __restrict__ part, int nblk, float* __restrict__ loss) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+  // staged by all threads (the loop's loads would each wait for memory), added in order by one
+  __shared__ float sp[2 * LOSS_BLOCKS];
+  for (int b = threadIdx.x; b < 2 * nblk; b += blockDim.x) sp[b] = part[b];
+  __syncthreads();
+  if (threadIdx.x != 0) return;
   float a = 0.f, m = 0.f;
-  for (int b = 0; b < nblk; ++b) { a = a + part[2 * b]; m = m + part[2 * b + 1]; }
+  for (int b = 0; b < nblk; ++b) { a = a + sp[2 * b]; m = m + sp[2 * b + 1]; }
   loss[0] = m > 0.f ? a / m : 0.f;
   loss[1] = m;
 }
@@ -1051,12 +1177,11 @@ bool activation_map(CUtensorMap* m, const bf16* x, int B, int H, int W) {
 int forward(const Workspace& ws, const float* params, const float* feat, int B, int H, int W, float* out,
             cudaStream_t st) {
   const float* bias0 = params + OFF_BLK + 9 * C * C;
-  const dim3 grid = tiles(B, H, W);
+  const dim3 grid((W + ST_W - 1) / ST_W, (H + TH - 1) / TH, B);
   CUtensorMap maps[SI3D_NET_BLOCKS];
   for (int k = 0; k < SI3D_NET_BLOCKS; ++k)
     if (!activation_map(&maps[k], ws.training ? ws.x[k] : ws.x[k & 1], B, H, W)) return SI3D_ECUDA;
-  k_stem<<<dim3((W + ST_W - 1) / ST_W, (H + TH - 1) / TH, B), TP, 0, st>>>(feat, ws.stem, H, W, ws.x[0],
-                                                                         ws.training ? ws.y[0] : nullptr);
+  k_stem<<<grid, 32 * TH, 0, st>>>(feat, ws.stem, H, W, ws.x[0], ws.training ? ws.y[0] : nullptr);
   const int nb = conv_tc_blocks(B, H, W);
   for (int k = 0; k < SI3D_NET_BLOCKS; ++k) {
     bf16* xout = ws.training ? ws.x[k + 1] : ws.x[(k + 1) & 1];
@@ -1065,7 +1190,7 @@ int forward(const Workspace& ws, const float* params, const float* feat, int B, 
                                                   ws.training ? ws.y[k + 1] : nullptr);
   }
   const bf16* xl = ws.training ? ws.x[SI3D_NET_BLOCKS] : ws.x[SI3D_NET_BLOCKS & 1];
-  k_head<<<grid, TP, 0, st>>>(xl, ws.head, H, W, out);
+  k_head<<<grid, HD_T, 0, st>>>(xl, ws.head, H, W, out);
   return 0;
 }
 
@@ -1078,7 +1203,7 @@ void backward(const Workspace& ws, const float* feat, const float* gout, int B, 
   k_head_bwd<<<grid, TP, 0, st>>>(gout, ws.head, H, W, ws.y[SI3D_NET_BLOCKS], ws.G, ws.DY, ws.DYb[0]);
   const int nb = conv_bwd_blocks(B, H, W);
   for (int k = SI3D_NET_BLOCKS - 1, cur = 0; k >= 0; --k, cur ^= 1) {
-    k_wgrad<C, C, bf16><<<WG_BLOCKS, 32 * WGW, 0, st>>>(ws.x[k], ws.DY, B, H, W, ws.part);
+    k_wgrad32<<<WG_BLOCKS, GT, 0, st>>>(ws.x[k], ws.DY, B, H, W, ws.part);
     k_wgrad_reduce<<<(BLK_SZ + 31) / 32, dim3(32, WR), 0, st>>>(ws.part, WG_BLOCKS, BLK_SZ, grad + OFF_BLK + k * BLK_SZ);
     k_conv32_bwd<<<nb, 128, 0, st>>>(ws.DYb[cur], ws.wbwd + (size_t)k * 9 * C * C, B, H, W, ws.G, ws.y[k], ws.DY,
                                      k > 0 ? ws.DYb[cur ^ 1] : nullptr);
@@ -1129,10 +1254,10 @@ int si3d_net_forward(const float* params, const float* feat, int B, int H, int W
 
 int si3d_net_loss(const float* out, const float* target, const float* mask, int n, float* gout, float* loss_dev) {
   if (!out || !target || !mask || !gout || !loss_dev || n < 1) return SI3D_EDIMS;
-  constexpr int NB = 148;
+  constexpr int NB = si3d::learn::LOSS_BLOCKS;
   float* part = loss_dev + 2;   // the caller's loss buffer holds 2 + 2 * 148 floats
   si3d::learn::k_loss_part<<<NB, 256>>>(out, target, mask, n, part);
-  si3d::learn::k_loss_final<<<1, 32>>>(part, NB, loss_dev);
+  si3d::learn::k_loss_final<<<1, 256>>>(part, NB, loss_dev);
   si3d::learn::k_loss_grad<<<(n + 255) / 256, 256>>>(out, target, mask, n, loss_dev, gout);
   return cudaGetLastError() == cudaSuccess ? SI3D_OK : SI3D_ECUDA;
 }
