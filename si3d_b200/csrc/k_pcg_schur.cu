@@ -18,7 +18,7 @@
 // What that buys: half the vectors, and two grid-wide exchanges an iteration instead of three, both
 // all-gather barriers that carry the dot products (coop.cuh).  A block owns consecutive black nodes
 // and keeps their coefficients, neighbour indices and vectors in shared memory for the whole solve.
-// Two forms share the arithmetic (the values are the same, bit for bit):
+// Three forms share the arithmetic (the values are the same, bit for bit):
 //   window  p of the block's nodes and of the `reach` nodes before and after them is in shared
 //           memory (reach: the largest index distance of two coupled nodes), so S p reads shared
 //           memory only.  A block publishes z as tagged words that carry their own arrival, like
@@ -26,10 +26,14 @@
 //           fence is needed in the iteration.
 //   stream  for blocks whose window does not fit: z and p go through L2, with fences at the
 //           exchange that follows their writes.
+//   cluster the window form for up to eight blocks: one thread-block cluster, whose blocks exchange
+//           sums and z through each other's shared memory, behind the cluster's barrier; a block has
+//           at most one node a thread, with its coefficients in registers.  3924 unknowns, four
+//           blocks: 4.5 -> 2.8 us an iteration.
 // Nodes beyond the shared-memory capacity keep their coefficients and vectors in global scratch.
 // The solve is bound by the latency of the two exchanges (about 1.2 us each) and of the FP64 chains
 // between them until a block holds about a thousand nodes.  Time of an iteration, two-colour loop ->
-// this loop: 3924 unknowns 13.0 -> 4.1 us, 129155 (FP32 inner solves) 13.3 -> 6.2 us with the
+// this loop: 3924 unknowns 13.0 -> 2.8 us, 129155 (FP32 inner solves) 13.3 -> 6.2 us with the
 // refinement around them, 350000 16.9 -> 5.9 us.
 #include <algorithm>
 #include <type_traits>
@@ -49,6 +53,7 @@ constexpr int SB = 512;    // threads per block (one block per SM); fixed, so th
                            // not depend on the launch it is solved in
 constexpr int RN = 3;      // nodes of a thread whose vectors are in registers (1536 of a block)
 constexpr int kSmemMax = 225 * 1024;
+constexpr int kClusterMax = 8;   // blocks of a cluster (the portable limit)
 
 // Shared memory of a node: nine coefficients and eight neighbours (16-bit in the window form).  The
 // vectors of a thread's first RN nodes are in its registers, those of later nodes in global memory.
@@ -90,29 +95,104 @@ __device__ __forceinline__ bool get_z(const uint4* zt, int j, float& z, unsigned
   return v.y == tag;
 }
 
-// One system, solved by the nb blocks that share `bar` and P.slots, this one being block bid.
-template <typename T, bool WIN>
+// Sums of v[] over all threads of the cluster's nb <= kClusterMax blocks, in every thread, in the order of
+// gather_sum (the same bits).  A block leaves its sums in its shared memory (tot: [2][kSlotVals], used in
+// turn), and after the cluster's barrier every warp reads all blocks'.  (Every warp reading the sums of
+// all warps of all blocks spares a reduction before the barrier, but reading other blocks' shared
+// memory is what takes the time: 925 us instead of 818 for 294 iterations.)  `then` loads what else
+// the barrier ordered.  The barrier also orders the shared and global memory of the blocks.  It needs no
+// limit: the blocks of a cluster run together, and all of them take the same path through the loop.
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned int in_block(const void* p, int block) {   // p's address in another block
+  unsigned int a = (unsigned int)__cvta_generic_to_shared(p);
+  asm volatile("mapa.shared::cluster.u32 %0, %0, %1;" : "+r"(a) : "r"(block));
+  return a;
+}
+__device__ __forceinline__ void ld_block(const double* p, int block, double& v) {
+  asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(in_block(p, block)) : "memory");
+}
+__device__ __forceinline__ void ld_block(const float* p, int block, float& v) {
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(in_block(p, block)) : "memory");
+}
+template <int NV, typename Then>
+__device__ __forceinline__ void cluster_sum(double (&v)[NV], int nb, int& turn, double* sh, double* tot, Then&& then) {
+  constexpr int NW = SB / 32;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] += __shfl_down_sync(0xffffffffu, v[i], o);
+  }
+  const int w = threadIdx.x >> 5, ln = threadIdx.x & 31;
+  if (ln == 0) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) sh[i * NW + w] = v[i];
+  }
+  __syncthreads();
+  double* const mine = tot + turn * kSlotVals;
+  turn ^= 1;
+  if (w == 0) {
+    double a[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) a[i] = ln < NW ? sh[i * NW + ln] : 0.0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) a[i] += __shfl_xor_sync(0xffffffffu, a[i], o);
+    }
+    if (ln == 0) {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) mine[i] = a[i];
+    }
+    __syncwarp();
+  }
+  cluster_barrier();
+  const int b = ln & (kClusterMax - 1);
+#pragma unroll
+  for (int i = 0; i < NV; ++i) {
+    v[i] = 0.0;
+    if (b < nb) ld_block(mine + i, b, v[i]);
+  }
+  then();
+#pragma unroll
+  for (int o = kClusterMax / 2; o > 0; o >>= 1) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) v[i] += __shfl_xor_sync(0xffffffffu, v[i], o);
+  }
+}
+
+// One system, solved by the nb blocks that share `bar` and P.slots, this one being block bid; CL: by the
+// nb blocks of a cluster (window form, every node in registers and shared memory), which exchange sums
+// and z through each other's shared memory.
+template <typename T, bool WIN, bool CL = false>
 __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, int bid, int nb, int smem) {
+  constexpr int RK = CL ? 1 : RN;   // (a cluster's block has at most SB nodes)
   using Idx = typename std::conditional<WIN, unsigned short, int>::type;
   extern __shared__ double dyn[];
   __shared__ double sh[2 * kSlotVals * SB / 32];
+  __shared__ double s_tot[2 * kSlotVals];
   const PcgColorT<T> &R = P.R, &B = P.B;
   PcgScal* SC = P.sc;
   if (SC->done != 0) return;
   const int nB = B.n, per = (nB + nb - 1) / nb, reach = P.reach;
   const int lo = min(bid * per, nB), n = min(per, nB - lo);
   const int wbytes = WIN ? (int)window_bytes<T>(per, reach) : 0;
-  const int cap = ((smem - wbytes) / node_bytes<T, WIN>()) & ~1, nres = min(n, cap);
+  const int zbytes = CL ? per * (int)sizeof(T) : 0;
+  const int cap = ((smem - wbytes - zbytes) / node_bytes<T, WIN>()) & ~1, nres = min(n, cap);
   // window entry of global node o: o - w0; entry wz is zero
   T* const s_w = reinterpret_cast<T*>(dyn);
   const int w0 = lo - reach, wz = per + 2 * reach;
   T* const s_h = s_w + wz + 1;   // z of the halo nodes
   T* const s_cf = reinterpret_cast<T*>(reinterpret_cast<char*>(dyn) + wbytes);   // [9][cap]
   Idx* const s_nb = reinterpret_cast<Idx*>(s_cf + 9 * cap);                      // [8][cap]
-  T rt[RN], ru[RN], rv[RN], rg[RN], rd[RN], rp[RN];   // t, u, S p, g, 1 / pivot, p
-  const int i0 = threadIdx.x, it = i0 + RN * SB;      // first node, first node past the registers
+  T* const s_z = reinterpret_cast<T*>(s_nb + 8 * cap);                           // CL: [per]
+  T rt[RK], ru[RK], rv[RK], rg[RK], rd[RK], rp[RK];   // t, u, S p, g, 1 / pivot, p
+  const int i0 = threadIdx.x, it = i0 + RK * SB;      // first node, first node past the registers
   const int hl = min(reach, lo), hr = min(reach, nB - lo - n);                   // halo nodes before and after
-  SlotBar bs = slot_bar(bar, P.slots, bid, nb, P.slot_blocks);
+  SlotBar bs{};
+  if (!CL) bs = slot_bar(bar, P.slots, bid, nb, P.slot_blocks);
+  int turn = 0;
   T* const z = B.z;
   unsigned int tag = 1;
   // z of the halo nodes into shared memory, by the warps that do not poll the barrier, while it waits
@@ -129,6 +209,18 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
     }
     return true;
   };
+  // The same from the blocks of the cluster, by the threads that will use it: a thread's first in a
+  // register, so that only its use waits for the load.
+  T zh = (T)0;
+  const int ho = (int)threadIdx.x < hl ? lo - hl + (int)threadIdx.x : lo + n + ((int)threadIdx.x - hl), hb = ho / per;
+  auto cluster_halo = [&]() {
+    if ((int)threadIdx.x < hl + hr) ld_block(s_z + (ho - hb * per), hb, zh);
+    for (int h = threadIdx.x + SB; h < hl + hr; h += SB) {
+      const int o = h < hl ? lo - hl + h : lo + n + (h - hl), b = o / per;
+      ld_block(s_z + (o - b * per), b, s_h[h]);
+    }
+  };
+  auto nothing = [] {};
   // ---- the Schur complement's rows, g and t = r_B + g of this block's nodes
   double v2[2] = {0.0, 0.0}, w2[2] = {0.0, 0.0};
   auto row = [&](int i, T& rt_, T& ru_, T& rg_, T& rd_) {
@@ -172,23 +264,24 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       else P.nb8[(size_t)m * nB + j] = x;
     }
     rt_ = t; ru_ = B.u[j]; rg_ = g; rd_ = d;
-    if (WIN) put_z(P.zt, j, zj, 1u);
+    if (CL) s_z[i] = zj;
+    else if (WIN) put_z(P.zt, j, zj, 1u);
     else z[j] = zj;
     v2[0] += (double)t * (double)zj;
     v2[1] += (double)rb * (double)rb;
   };
 #pragma unroll
-  for (int k = 0; k < RN; ++k) rt[k] = ru[k] = rv[k] = rg[k] = rd[k] = rp[k] = (T)0;
+  for (int k = 0; k < RK; ++k) rt[k] = ru[k] = rv[k] = rg[k] = rd[k] = rp[k] = (T)0;
 #pragma unroll 1
   for (int i = i0, k = 0; i < n; i += SB, ++k) {
     T t, u, g, d;
     row(i, t, u, g, d);
-    if (k >= RN) {
+    if (k >= RK) {
       B.r[lo + i] = t;
       B.q[lo + i] = g;
     }
 #pragma unroll
-    for (int m = 0; m < RN; ++m)
+    for (int m = 0; m < RK; ++m)
       if (k == m) { rt[m] = t; ru[m] = u; rg[m] = g; rd[m] = d; }
   }
   if (WIN)
@@ -198,12 +291,26 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
     w2[0] += r0 * r0 * (double)R.dinv[k];
     w2[1] += r0 * r0;
   }
-  if (!gather_sum<2, false, SB>(w2, bs, SC, sh)) return;
-  // (with a fence in both forms: after it no tagged word of an earlier solve is left)
-  if (!gather_sum<2, true, SB>(v2, bs, SC, sh)) return;
-  if (WIN) {   // the first halo, now that no word of an earlier solve is left
-    double none[1] = {0.0};
-    if (!gather_sum<1, false, SB>(none, bs, SC, sh, fetch_halo)) return;
+  if (CL) {
+    cluster_sum<2>(w2, nb, turn, sh, s_tot, nothing);
+    cluster_sum<2>(v2, nb, turn, sh, s_tot, cluster_halo);
+  } else {
+    if (!gather_sum<2, false, SB>(w2, bs, SC, sh)) return;
+    // (with a fence in both forms: after it no tagged word of an earlier solve is left)
+    if (!gather_sum<2, true, SB>(v2, bs, SC, sh)) return;
+    if (WIN) {   // the first halo, now that no word of an earlier solve is left
+      double none[1] = {0.0};
+      if (!gather_sum<1, false, SB>(none, bs, SC, sh, fetch_halo)) return;
+    }
+  }
+  // the cluster form's node: coefficients and neighbours in registers too
+  T cfr[9];
+  int nbr[8];
+  if (CL && i0 < n) {
+#pragma unroll
+    for (int m = 0; m < 9; ++m) cfr[m] = s_cf[m * cap + i0];
+#pragma unroll
+    for (int m = 0; m < 8; ++m) nbr[m] = s_nb[m * cap + i0];
   }
   const double gamma = w2[0], delta = w2[1];
   double alpha = SC->alpha, beta = SC->beta, rzdot = SC->rzdot, dkm1 = SC->dkm1, rho = 1.0, c = 0.0, rrt = 0.0;
@@ -229,10 +336,10 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
     if (WIN) {
       for (int h = threadIdx.x; h < hl + hr; h += SB) {
         const int x = (h < hl ? lo - hl + h : lo + n + (h - hl)) - w0;
-        s_w[x] = s_h[h] + bt * s_w[x];
+        s_w[x] = (CL && h < SB ? zh : s_h[h]) + bt * s_w[x];
       }
 #pragma unroll
-      for (int k = 0; k < RN; ++k) {
+      for (int k = 0; k < RK; ++k) {
         rp[k] = rt[k] * rd[k] + bt * rp[k];
         if (i0 + k * SB < n) s_w[reach + i0 + k * SB] = rp[k];
       }
@@ -244,7 +351,12 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       const int j = lo + i;
       T cf[9];
       int o[8];
-      if (i < nres) {
+      if (CL) {
+#pragma unroll
+        for (int m = 0; m < 9; ++m) cf[m] = cfr[m];
+#pragma unroll
+        for (int m = 0; m < 8; ++m) o[m] = nbr[m];
+      } else if (i < nres) {
 #pragma unroll
         for (int m = 0; m < 9; ++m) cf[m] = s_cf[m * cap + i];
 #pragma unroll
@@ -264,7 +376,7 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       return (ya + yb) + yc;
     };
 #pragma unroll
-    for (int k = 0; k < RN; ++k) {
+    for (int k = 0; k < RK; ++k) {
       const int i = i0 + k * SB;
       if (i < n) {
         if (!WIN) {
@@ -282,12 +394,12 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       P.sv[lo + i] = y;
       pq[0] += (double)pi * (double)y;
     }
-    if (!gather_sum<1, false, SB>(pq, bs, SC, sh)) return;
+    if (CL) cluster_sum<1>(pq, nb, turn, sh, s_tot, nothing);
+    else if (!gather_sum<1, false, SB>(pq, bs, SC, sh)) return;
     c = rho + beta * c;
     const double pap = pq[0] + c * c * gamma;
     alpha = rzdot / pap;
     if (!(pap > 0.0)) { ier = -6; break; }
-    if (bid == 0 && threadIdx.x == 0 && in < hist_cap) { P.hist_alpha[in] = alpha; P.hist_beta[in] = beta; }
     in += 1;
     par ^= 1;
     ++tag;
@@ -297,13 +409,14 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
     v2[0] = v2[1] = 0.0;
     auto take = [&](int i, T t, T g, T d) {
       const T zj = t * d, rb = t - rh * g;
-      if (WIN) put_z(P.zt, lo + i, zj, tag);
+      if (CL) s_z[i] = zj;
+      else if (WIN) put_z(P.zt, lo + i, zj, tag);
       else z[lo + i] = zj;
       v2[0] += (double)t * (double)zj;
       v2[1] += (double)rb * (double)rb;
     };
 #pragma unroll
-    for (int k = 0; k < RN; ++k) {
+    for (int k = 0; k < RK; ++k) {
       rt[k] = rt[k] - al * rv[k];
       if (i0 + k * SB < n) take(i0 + k * SB, rt[k], rg[k], rd[k]);
       ru[k] = ru[k] + al * rp[k];
@@ -315,14 +428,22 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       B.u[j] = B.u[j] + al * (WIN ? s_w[reach + i] : pn[j]);
       take(i, t, B.q[j], B.dinv[j]);
     }
-    if (!gather_sum<2, !WIN, SB>(v2, bs, SC, sh, fetch_halo)) return;
+    if (CL) cluster_sum<2>(v2, nb, turn, sh, s_tot, cluster_halo);
+    else if (!gather_sum<2, !WIN, SB>(v2, bs, SC, sh, fetch_halo)) return;
+    // (here, far from the next exchange: the cluster's barrier waits for stores under way)
+    if (bid == 0 && threadIdx.x == 0 && in <= hist_cap) { P.hist_alpha[in - 1] = alpha; P.hist_beta[in - 1] = beta; }
   }
   // ---- u of the black nodes, then of the red nodes: D u_R = b_R - rho r0_R + C u_B (b = r0 from u = 0)
 #pragma unroll
-  for (int k = 0; k < RN; ++k)
+  for (int k = 0; k < RK; ++k)
     if (i0 + k * SB < n) B.u[lo + i0 + k * SB] = ru[k];
   double done[1] = {0.0};
-  if (!gather_sum<1, true, SB>(done, bs, SC, sh)) return;
+  if (CL) {
+    __threadfence();
+    cluster_barrier();   // (also: no block leaves while another may read its sums)
+  } else if (!gather_sum<1, true, SB>(done, bs, SC, sh)) {
+    return;
+  }
   const T rh = (T)rho;
   for (int k = bid * SB + threadIdx.x; k < R.n; k += nb * SB) {
     const int4 q = R.nbr[k];
@@ -352,6 +473,11 @@ __device__ __forceinline__ void schur_any(const PcgDevT<T>& P, GridBar* bar, int
 template <typename T>
 __global__ void __launch_bounds__(SB, 1) k_schur_loop(PcgDevT<T> P, GridBar* bar, int smem) {
   schur_any<T>(P, bar, blockIdx.x, gridDim.x, smem);
+}
+
+template <typename T>
+__global__ void __launch_bounds__(SB, 1) k_schur_cluster(PcgDevT<T> P, int smem) {
+  schur_body<T, true, true>(P, nullptr, blockIdx.x, gridDim.x, smem);
 }
 
 // The FP64 loops of an ensemble's basins in one cooperative launch: basin m's system is solved by
@@ -388,6 +514,27 @@ int coop_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int nblocks,
 
 template <typename T>
 int launch_schur(const PcgDevT<T>& P, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init) {
+  const int per = (P.B.n + nblocks - 1) / nblocks;
+  const int pe = (std::max(per, 2) + 1) / 2 * 2;
+  const long long win = window_bytes<T>(per, P.reach) + (long long)pe * node_bytes<T, true>();
+  // Up to eight blocks (4096 nodes) run as one cluster, when all of a block fits its shared memory; the
+  // test hook of the barriers' limit keeps to the grid's barriers.  More blocks than the portable cluster
+  // size have the grid's exchanges.
+  if (nblocks > 1 && nblocks <= kClusterMax && per <= SB && !init && win + (long long)per * (int)sizeof(T) <= kSmemMax) {
+    const int smem = (int)(win + (long long)per * (int)sizeof(T));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(nblocks);
+    cfg.blockDim = dim3(SB);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = nblocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_schur_cluster<T>, P, smem) == cudaSuccess ? 0 : -1;
+  }
   if (init) {
     if (cudaMemcpyAsync(bar, init, sizeof(GridBar), cudaMemcpyHostToDevice, st) != cudaSuccess) return -1;
   } else if (cudaMemsetAsync(bar, 0, sizeof(GridBar), st) != cudaSuccess) {
@@ -395,11 +542,7 @@ int launch_schur(const PcgDevT<T>& P, GridBar* bar, int nblocks, cudaStream_t st
   }
   const size_t pitch = sizeof(uint4) * (size_t)slot_plane(P.slot_blocks);
   if (cudaMemset2DAsync(P.slots, pitch, 0, sizeof(uint4) * (size_t)nblocks, 2 * kSlotVals, st) != cudaSuccess) return -1;
-  const int per = (P.B.n + nblocks - 1) / nblocks;
-  const int pe = (std::max(per, 2) + 1) / 2 * 2;
-  const int smem = (int)std::min<long long>(kSmemMax, window_fits<T>(per, P.reach)
-                                                          ? window_bytes<T>(per, P.reach) + (long long)pe * node_bytes<T, true>()
-                                                          : (long long)pe * node_bytes<T, false>());
+  const int smem = (int)std::min<long long>(kSmemMax, window_fits<T>(per, P.reach) ? win : (long long)pe * node_bytes<T, false>());
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
   coop_config(cfg, attr, nblocks, smem, st);
@@ -411,6 +554,8 @@ int launch_schur(const PcgDevT<T>& P, GridBar* bar, int nblocks, cudaStream_t st
 int schur_init() {
   if (cudaFuncSetAttribute(k_schur_loop<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
       cudaFuncSetAttribute(k_schur_loop<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
+      cudaFuncSetAttribute(k_schur_cluster<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
+      cudaFuncSetAttribute(k_schur_cluster<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess ||
       cudaFuncSetAttribute(k_schur_loop_ens, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax) != cudaSuccess)
     return -1;
   return 0;
