@@ -19,7 +19,7 @@
 //   coarse  black half-sweep of the coarsest level
 //   up      per level k = L - 2 .. 0: black half-sweep with the neighbours' values plus the coarse
 //           correction of their aggregate; red half-sweep; at level 0 both add to (r, z).  The
-//           red half-sweeps of the coarsest level and of levels >= 2 are not run as phases: the
+//           red half-sweeps of the coarsest level and of levels >= 2 (small systems: 1) are not run: the
 //           black half-sweep of the next finer level forms each red aggregate it reads from that
 //           aggregate's black neighbours (the same expression, so the same values)
 //   PQ      beta, p = z + beta p and q = A p (neighbours' p formed on the fly), (p, q)
@@ -62,8 +62,10 @@ constexpr int UG = 2;                 // groups of four cells a thread keeps in 
 constexpr int UH = 2;                 // groups in flight in the half-sweeps
 // Levels from kSweptFrom on (and the coarsest) skip their red half-sweep of the way up: the finer
 // level's black half-sweep forms the red values it reads from their black neighbours (swept_z).
-// Cheap on the small levels, it saves a grid barrier a level; on levels 0 and 1 the recomputation
-// costs more than the barrier.
+// Cheap on the small levels, it saves a grid barrier a level.  On level 1 it pays while level 0 is one
+// pass of the grid's threads, a group each (517 x 283: 2968 -> 2904 us a step, 640 x 360: 5411 -> 5370;
+// 2000 x 1000, seven passes: 21.43 -> 21.55 ms).  The black half-sweep of the way down on level 1 or 0
+// formed by the restriction costs as much as its barrier at all of these.
 constexpr int kSweptFrom = 2;
 constexpr int kSpreadFrom = 2;   // levels whose items are dealt round robin (first_item_spread)
 constexpr int MQ = 512;               // threads per block of the cooperative solve (one block per SM)
@@ -365,6 +367,7 @@ __device__ bool mg_pcg(const MgDev& M, const MgLevel* s_lv, int nlev, GridBar* b
   ier = 0;
   const MgLevel& L0 = s_lv[0];
   const int n0q = L0.rows * L0.nq, pt = L0.pitch;
+  const int up_from = n0q <= stride ? 1 : kSweptFrom;   // levels without a red half-sweep on the way up
   for (;;) {
     // ---- U: u += alpha p, r -= alpha q; (r, r); z = dinv r, the red half-sweep of level 0 from zero
     // (written for the black cells too: the black half-sweep replaces them before they are read)
@@ -433,10 +436,10 @@ __device__ bool mg_pcg(const MgDev& M, const MgLevel* s_lv, int nlev, GridBar* b
     half_sweep<false, false, UH>(s_lv[nlev - 1], s_lv[nlev - 1], 1, gk(nlev - 1), stride);
     if (!grid_barrier(bar, SC, s_flag)) return false;
     // ---- up: black half-sweep with the coarse correction, red half-sweep; (r, z) at level 0.  The
-    // red half-sweeps of levels >= kSweptFrom (and of the coarsest) are not run: the black half-sweep
+    // red half-sweeps of levels >= up_from (and of the coarsest) are not run: the black half-sweep
     // of the next finer level forms the red aggregates it reads (swept_z), one barrier fewer each.
     for (int k = nlev - 2; k >= 0; --k) {
-      const bool swept = k + 1 >= kSweptFrom || k + 1 == nlev - 1;
+      const bool swept = k + 1 >= up_from || k + 1 == nlev - 1;
       if (k == 0) {
         double w[1] = {swept ? half_sweep<true, true, 1, true>(s_lv[0], s_lv[1], 1, g0, stride)
                              : half_sweep<true, true, UH>(s_lv[0], s_lv[1], 1, g0, stride)};
@@ -448,7 +451,7 @@ __device__ bool mg_pcg(const MgDev& M, const MgLevel* s_lv, int nlev, GridBar* b
         half_sweep<true, false, UH>(s_lv[k], s_lv[k + 1], 1, gk(k), stride);
       }
       if (!grid_barrier(bar, SC, s_flag)) return false;
-      if (k >= kSweptFrom) continue;
+      if (k >= up_from) continue;
       if (k == 0) {
         double w[1] = {half_sweep<false, true, UH>(s_lv[0], s_lv[0], 0, g0, stride)};
         bsum<1, MQ>(w, sh);
