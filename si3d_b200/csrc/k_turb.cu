@@ -77,9 +77,14 @@ __global__ void __launch_bounds__(32 * CLN) k_turb_cells(Dev d, TurbConst T, dou
 __global__ void k_turb_column(Dev d, TurbConst T, double* __restrict__ sxl, double* __restrict__ ssp,
                               double* __restrict__ sbp, double* __restrict__ szb, double* __restrict__ se) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x + 1;
-  if (l > d.g.lm) return;
-  const int kms = NB(d.g.kmz, l), k1s = d.s.k1z[l - 1], k1 = d.g.k1, km1 = d.g.km1, P = d.g.P;
-  if (kms - k1s + 1 <= 1) return;
+  const bool in = l <= d.g.lm;
+  const int kms = in ? NB(d.g.kmz, l) : 0, k1s = in ? d.s.k1z[l - 1] : 1, k1 = d.g.k1, km1 = d.g.km1, P = d.g.P;
+  const bool on = in && kms - k1s + 1 > 1;
+  // the warp's deepest layer: the sweeps from the bottom start there for all lanes, so that a warp's
+  // accesses stay in one layer (each from its own bottom, they would be in up to 32): 212 -> 192 us at
+  // 640 x 360 x 45, with the backward sweeps' loads four layers at a time
+  const int kmw = __reduce_max_sync(0xffffffffu, on ? kms : 0);
+  if (!on) return;
   const int lW = NB(d.g.lWC, l), lS = NB(d.g.lSC, l), dW = lW - l, dS = lS - l;
   const double twodt1 = d.p.twodt * d.tz;   // twodt / istep
   const double* __restrict__ hp = d.f.hp;
@@ -96,7 +101,19 @@ __global__ void k_turb_column(Dev d, TurbConst T, double* __restrict__ sxl, doub
   // ---- distances from the bottom (summed from the bottom up, as the reference does)
   {
     double z0 = 0.0;
-    for (int k = kms; k >= k1s + 1; --k) { z0 = z0 + hp[IX(d, k, l)]; szb[IX(d, k, l)] = z0; }
+    for (int k0 = kmw; k0 >= k1s + 1; k0 -= 4) {
+      double h[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 - i;
+        h[i] = (k <= kms && k >= k1s + 1) ? hp[IX(d, k, l)] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 - i;
+        if (k <= kms && k >= k1s + 1) { z0 = z0 + h[i]; szb[IX(d, k, l)] = z0; }
+      }
+    }
   }
   if (hp[IX(d, k1s, l)] < 1.E-2) {
     const int ik = IX(d, k1s + 1, l);
@@ -104,7 +121,7 @@ __global__ void k_turb_column(Dev d, TurbConst T, double* __restrict__ sxl, doub
     Dv[ik] = fmax(Dv[ik], 1.E-4);
   }
   for (int k = 1; k <= k1s; ++k) { Av[IX(d, k, l)] = 0.0; Dv[IX(d, k, l)] = 0.0; }
-  for (int k = kms + 1; k <= km1; ++k) { Av[IX(d, k, l)] = 0.0; Dv[IX(d, k, l)] = 0.0; }
+  for (int k = km1; k >= kms + 1; --k) { Av[IX(d, k, l)] = 0.0; Dv[IX(d, k, l)] = 0.0; }
   // ---- boundary values: bottom and surface friction velocities squared
   const int ikb = IX(d, kms, l);
   const double ub = 0.5 * (d.f.u[ikb] + d.f.u[ikb + dW]), vb = 0.5 * (d.f.v[ikb] + d.f.v[ikb + dS]);
@@ -187,17 +204,27 @@ __global__ void k_turb_column(Dev d, TurbConst T, double* __restrict__ sxl, doub
     double x0 = f0, x1 = f1;
     q2[IX(d, kms + 1, l)] = fmax(kQ2Min, x0);
     q2l[IX(d, kms + 1, l)] = fmax(kQ2lMin, x1);
-    // backward sweeps, the next layer's factors and forward values loaded ahead
-    double en0 = se[IX(d, kms, l)], fn0 = q2[IX(d, kms, l)];
-    double en1 = ssp[IX(d, kms, l)], fn1 = q2l[IX(d, kms, l)];
-    for (int k = kms; k >= k1s; --k) {
-      const int ik = IX(d, k, l);
-      const double ea = en0, fa = fn0, eb = en1, fb = fn1;
-      if (k - 1 >= k1s) { en0 = se[ik - P]; fn0 = q2[ik - P]; en1 = ssp[ik - P]; fn1 = q2l[ik - P]; }
-      x0 = ea * x0 + fa;
-      q2[ik] = fmax(kQ2Min, x0);
-      x1 = eb * x1 + fb;
-      q2l[ik] = fmax(kQ2lMin, x1);
+    // backward sweeps, four layers' factors and forward values loaded together
+    for (int k0 = kmw; k0 >= k1s; k0 -= 4) {
+      double e0v[4], f0v[4], e1v[4], f1v[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 - i;
+        const bool ok = k <= kms && k >= k1s;
+        const int ik = IX(d, k, l);
+        e0v[i] = ok ? se[ik] : 0.0; f0v[i] = ok ? q2[ik] : 0.0;
+        e1v[i] = ok ? ssp[ik] : 0.0; f1v[i] = ok ? q2l[ik] : 0.0;
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int k = k0 - i;
+        if (k > kms || k < k1s) continue;
+        const int ik = IX(d, k, l);
+        x0 = e0v[i] * x0 + f0v[i];
+        q2[ik] = fmax(kQ2Min, x0);
+        x1 = e1v[i] * x1 + f1v[i];
+        q2l[ik] = fmax(kQ2lMin, x1);
+      }
     }
     const double top0 = q2[IX(d, k1s, l)], top1 = q2l[IX(d, k1s, l)];
     for (int k = k1; k <= k1s - 1; ++k) { q2[IX(d, k, l)] = top0; q2l[IX(d, k, l)] = top1; }
@@ -209,11 +236,25 @@ __global__ void k_turb_half(Dev d, int mode) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (l > d.g.lm) return;
   const int kms = NB(d.g.kmz, l), k1s = d.s.k1z[l - 1], P = d.g.P;
-  for (int k = d.g.k1; k <= kms; ++k) {
-    const int ik = IX(d, k, l);
-    if (mode == 1) { d.f.q2pp[ik] = d.f.q2p[ik]; d.f.q2lpp[ik] = d.f.q2lp[ik]; }
-    d.f.q2p[ik] = 0.5 * (d.f.q2[ik] + d.f.q2pp[ik]);
-    d.f.q2lp[ik] = 0.5 * (d.f.q2l[ik] + d.f.q2lpp[ik]);
+  // four layers' loads in flight together (79 -> 27 us at 640 x 360 x 45)
+  for (int k0 = d.g.k1; k0 <= kms; k0 += 4) {
+    double a[4], b[4], ao[4], bo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (k0 + i > kms) continue;
+      const int ik = IX(d, k0 + i, l);
+      a[i] = d.f.q2[ik]; b[i] = d.f.q2l[ik];
+      ao[i] = mode == 1 ? d.f.q2p[ik] : d.f.q2pp[ik];
+      bo[i] = mode == 1 ? d.f.q2lp[ik] : d.f.q2lpp[ik];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (k0 + i > kms) continue;
+      const int ik = IX(d, k0 + i, l);
+      if (mode == 1) { d.f.q2pp[ik] = ao[i]; d.f.q2lpp[ik] = bo[i]; }
+      d.f.q2p[ik] = 0.5 * (a[i] + ao[i]);
+      d.f.q2lp[ik] = 0.5 * (b[i] + bo[i]);
+    }
   }
   if (k1s + 2 <= d.g.km1 && d.f.hpp[IX(d, k1s, l)] <= ZERO) {
     const int ik = IX(d, k1s + 1, l);
@@ -228,18 +269,31 @@ __global__ void k_turb_save(Dev d, int istep) {
   const int l = blockIdx.x * blockDim.x + threadIdx.x + 1;
   if (l > d.g.lm1) return;
   const int km1 = d.g.km1, P = d.g.P;
-  for (int k = 1; k <= km1; ++k) {
-    const int ik = IX(d, k, l);
-    if (istep == 1) { d.f.q2pp[ik] = d.f.q2p[ik]; d.f.q2lpp[ik] = d.f.q2lp[ik]; }
-    d.f.q2p[ik] = d.f.q2[ik];
-    d.f.q2lp[ik] = d.f.q2l[ik];
+  // four layers' loads in flight together (112 -> 78 us at 640 x 360 x 45)
+  const bool wet = l <= d.g.lm;
+  for (int k0 = 1; k0 <= km1; k0 += 4) {
+    double a[4], b[4], u[4], v[4], ao[4], bo[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = k0 + i;
+      if (k > km1) continue;
+      const int ik = IX(d, k, l);
+      a[i] = d.f.q2[ik]; b[i] = d.f.q2l[ik];
+      if (istep == 1) { ao[i] = d.f.q2p[ik]; bo[i] = d.f.q2lp[ik]; }
+      if (wet && k >= d.g.k1 && k <= d.g.km) { u[i] = d.f.up[ik]; v[i] = d.f.vp[ik]; }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int k = k0 + i;
+      if (k > km1) continue;
+      const int ik = IX(d, k, l);
+      if (istep == 1) { d.f.q2pp[ik] = ao[i]; d.f.q2lpp[ik] = bo[i]; }
+      d.f.q2p[ik] = a[i];
+      d.f.q2lp[ik] = b[i];
+      if (wet && k >= d.g.k1 && k <= d.g.km) { d.f.u[ik] = u[i]; d.f.v[ik] = v[i]; }
+    }
   }
-  if (l > d.g.lm) return;
-  for (int k = d.g.k1; k <= d.g.km; ++k) {
-    const int ik = IX(d, k, l);
-    d.f.u[ik] = d.f.up[ik];
-    d.f.v[ik] = d.f.vp[ik];
-  }
+  if (!wet) return;
   const int k1s = d.s.k1z[l - 1];
   if ((istep == 1 || km1 - k1s > 1) && k1s + 2 <= km1 && d.f.hpp[IX(d, k1s, l)] <= ZERO) {
     const int ik = IX(d, k1s + 1, l);
