@@ -163,11 +163,13 @@ __device__ __forceinline__ void cluster_sum(double (&v)[NV], int nb, int& turn, 
 }
 
 // One system, solved by the nb blocks that share `bar` and P.slots, this one being block bid; CL: by the
-// nb blocks of a cluster (window form, every node in registers and shared memory), which exchange sums
-// and z through each other's shared memory.
-template <typename T, bool WIN, bool CL = false>
+// nb blocks of a cluster (window form, ONE), which exchange sums and z through each other's shared
+// memory.  ONE: at most one node a thread, all of the block's in shared memory (window form); its
+// coefficients are read from registers, which takes 630 instead of 1180 cycles for S p of 491 nodes
+// (129,155 unknowns in FP32, 436 nodes a block: 2.81 -> 2.60 ms of solves a step).
+template <typename T, bool WIN, bool ONE, bool CL = false>
 __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, int bid, int nb, int smem) {
-  constexpr int RK = CL ? 1 : RN;   // (a cluster's block has at most SB nodes)
+  constexpr int RK = ONE ? 1 : RN;
   using Idx = typename std::conditional<WIN, unsigned short, int>::type;
   extern __shared__ double dyn[];
   __shared__ double sh[2 * kSlotVals * SB / 32];
@@ -303,10 +305,10 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       if (!gather_sum<1, false, SB>(none, bs, SC, sh, fetch_halo)) return;
     }
   }
-  // the cluster form's node: coefficients and neighbours in registers too
+  // ONE: the thread's node's coefficients and neighbours in registers too
   T cfr[9];
   int nbr[8];
-  if (CL && i0 < n) {
+  if (ONE && i0 < n) {
 #pragma unroll
     for (int m = 0; m < 9; ++m) cfr[m] = s_cf[m * cap + i0];
 #pragma unroll
@@ -351,7 +353,7 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
       const int j = lo + i;
       T cf[9];
       int o[8];
-      if (CL) {
+      if (ONE) {
 #pragma unroll
         for (int m = 0; m < 9; ++m) cf[m] = cfr[m];
 #pragma unroll
@@ -466,8 +468,11 @@ __device__ __forceinline__ void schur_body(const PcgDevT<T>& P, GridBar* bar, in
 // The form depends on the nodes per block and the reach alone, so every block of a system takes the same.
 template <typename T>
 __device__ __forceinline__ void schur_any(const PcgDevT<T>& P, GridBar* bar, int bid, int nb, int smem) {
-  if (window_fits<T>((P.B.n + nb - 1) / nb, P.reach)) schur_body<T, true>(P, bar, bid, nb, smem);
-  else schur_body<T, false>(P, bar, bid, nb, smem);
+  const int per = (P.B.n + nb - 1) / nb;
+  const long long all = window_bytes<T>(per, P.reach) + (long long)((per + 1) / 2 * 2) * node_bytes<T, true>();
+  if (per <= SB && all <= smem) schur_body<T, true, true>(P, bar, bid, nb, smem);
+  else if (window_fits<T>(per, P.reach)) schur_body<T, true, false>(P, bar, bid, nb, smem);
+  else schur_body<T, false, false>(P, bar, bid, nb, smem);
 }
 
 template <typename T>
@@ -477,7 +482,7 @@ __global__ void __launch_bounds__(SB, 1) k_schur_loop(PcgDevT<T> P, GridBar* bar
 
 template <typename T>
 __global__ void __launch_bounds__(SB, 1) k_schur_cluster(PcgDevT<T> P, int smem) {
-  schur_body<T, true, true>(P, nullptr, blockIdx.x, gridDim.x, smem);
+  schur_body<T, true, true, true>(P, nullptr, blockIdx.x, gridDim.x, smem);
 }
 
 // The FP64 loops of an ensemble's basins in one cooperative launch: basin m's system is solved by
