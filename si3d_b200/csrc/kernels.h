@@ -158,7 +158,7 @@ void nat_setup(const Dev& d, const NatDev& N, int x0_mode, const double* dz, cud
 int nat_solve(const NatDev& N, bool test2, cudaStream_t st);
 void nat_finish(const Dev& d, const NatDev& N, cudaStream_t st);
 // `init` (host memory, optional) replaces the zeroed barrier record of this launch
-// One basin's share of an ensemble's batched FP64 solve (k_pcg_loop_ens): its system, its own
+// One basin's share of an ensemble's batched FP64 solve (k_schur_loop_ens): its system, its own
 // barrier record, and the blocks [first, first + nblk) of the launch that solve it.
 struct PcgEnsItem {
   PcgDev P;

@@ -2231,7 +2231,7 @@ static int ens_upload_shares(Ens* E, const std::vector<std::vector<double>>* its
 
 // Capture one step (n >= 2) with every zeta solve batched: the members advance in lock step on their
 // own streams up to each solve's set-up, join the master stream for one cooperative launch that
-// solves all of their systems (k_pcg_loop_ens, each member on its share of the blocks with its own
+// solves all of their systems (k_schur_loop_ens, each member on its share of the blocks with its own
 // barrier record), and fork again for the rest of the fd call.  The stage sequence is step_impl's
 // for n >= 2.  The k-th launch reads its shares from slot k of the item array, which the steps
 // refresh from each solve's last iteration counts without capturing again.
