@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/si3d_gpu.h"
 #include "../../include/si3d_learn.h"
@@ -664,7 +665,13 @@ constexpr int GHP = (GH + 2) * WT;         // with frame
 // pixels): 0.7e-7 to 1.7e-7, of FP32 multiply-adds 1.1e-7 to 3.9e-7; with one chain a tile or a block it
 // would be up to 3 times that of FP32.  32 x 64 x 64 pixels, per call: FP32 cores, one load a multiply-add
 // 200 us; FP32 cores, 9 x 4 sums a thread 66 (9 x 8: 67, packed pairs: 65; bound by the FP32 pipes); this: 32.
-// An infinite DY gives infinities (its lower terms are zero), except against an infinite X: NaN.
+// Two kinds of values need more, and a block that meets one walks its tiles a second time in the WIDE form
+// (looking out for them takes 1.7 us a call, the WIDE form at once would take 7.5 us):
+//   a DY below kTiny, whose lower terms would fall below BF16's range: in the WIDE form a term is held 2^7
+//   times as large as its part of DY, once for the second and twice for the third, and the sums are scaled
+//   back between the terms.  2^7 and no more, so that no term is larger than the one before;
+//   an infinite X, which gives NaN against a lower term that is zero where DY is not: in the WIDE form the
+//   lower terms meet X without its infinities.  (The lower terms of an infinite DY are zero.)
 constexpr int GT = 9 * 32;                 // threads: a warp a tap
 __device__ __forceinline__ void ldsm4t(uint32_t* r, const bf16* p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
@@ -675,6 +682,8 @@ __device__ __forceinline__ uint32_t top_halves(float a, float b) {   // two FP32
 }
 __device__ __forceinline__ float cut(float a) { return __uint_as_float(__float_as_uint(a) & 0xffff0000u); }
 __device__ __forceinline__ float rest(float a) { return isinf(a) ? 0.f : a - cut(a); }   // exact
+constexpr uint32_t kTiny = (127u - 100u) << 23;   // 2^-100: its third term's last bit is 2^-123, a normal number
+__device__ __forceinline__ uint32_t magnitude(float a) { return (__float_as_uint(a) << 1) - 1u; }   // zero: the largest
 
 __global__ void __launch_bounds__(GT, 2) k_wgrad32(const bf16* __restrict__ X, const float* __restrict__ DY, int B, int H,
                                                    int W, float* __restrict__ part) {
@@ -685,13 +694,7 @@ __global__ void __launch_bounds__(GT, 2) k_wgrad32(const bf16* __restrict__ X, c
   const int nj = (W + TW - 1) / TW, ni = (H + GH - 1) / GH, ntiles = B * ni * nj;
   const int c4 = threadIdx.x % (C / 4) * 4;        // the channels it stages (GT is a multiple of 8)
   float acc[2][4][4];                              // [ci / 16][co / 8][fragment]
-#pragma unroll
-  for (int m = 0; m < 2; ++m)
-#pragma unroll
-    for (int n = 0; n < 4; ++n)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
-  float4 sum = make_float4(0.f, 0.f, 0.f, 0.f), rd[ND];
+  float4 sum, rd[ND];
   auto fetch = [&](int tile, int buf) {
     const int b = tile / (ni * nj), rem = tile - b * (ni * nj), i0 = rem / nj * GH, j0 = rem % nj * TW;
     stage_tile<GH + 2, WT, GT>(sX[buf], X, b, i0, j0, H, W);
@@ -703,60 +706,93 @@ __global__ void __launch_bounds__(GT, 2) k_wgrad32(const bf16* __restrict__ X, c
         rd[k] = *reinterpret_cast<const float4*>(DY + (((size_t)b * H + gi) * W + gj) * C + c4);
     }
   };
-  int buf = 0;
-  if ((int)blockIdx.x < ntiles) fetch(blockIdx.x, 0);
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
-    __syncthreads();   // the previous tile's readers are done
+  auto walk = [&](auto form) -> bool {   // whether it met a value that needs the WIDE form
+    constexpr bool WIDE = decltype(form)::value;
+    uint32_t least = 0xffffffffu;
+    int buf = 0;
 #pragma unroll
-    for (int k = 0; k < ND; ++k) {
-      const int pix = (threadIdx.x + k * GT) / (C / 4);
-      float4 d = rd[k];
-      sum.x = sum.x + d.x; sum.y = sum.y + d.y; sum.z = sum.z + d.z; sum.w = sum.w + d.w;
-      if (pix < GP) {
+    for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int s = 0; s < 3; ++s) {
-          *reinterpret_cast<uint2*>(&sD[s][pix * XS + c4]) = make_uint2(top_halves(d.x, d.y), top_halves(d.z, d.w));
-          d = make_float4(rest(d.x), rest(d.y), rest(d.z), rest(d.w));
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) acc[m][n][e] = 0.f;
+    sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    if ((int)blockIdx.x < ntiles) fetch(blockIdx.x, 0);
+    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x, buf ^= 1) {
+      __syncthreads();   // the previous tile's readers are done
+#pragma unroll
+      for (int k = 0; k < ND; ++k) {
+        const int pix = (threadIdx.x + k * GT) / (C / 4);
+        float4 d = rd[k];
+        sum.x = sum.x + d.x; sum.y = sum.y + d.y; sum.z = sum.z + d.z; sum.w = sum.w + d.w;
+        if (!WIDE) least = min(min(least, min(magnitude(d.x), magnitude(d.y))), min(magnitude(d.z), magnitude(d.w)));
+        if (pix < GP) {
+#pragma unroll
+          for (int s = 0; s < 3; ++s) {
+            *reinterpret_cast<uint2*>(&sD[s][pix * XS + c4]) = make_uint2(top_halves(d.x, d.y), top_halves(d.z, d.w));
+            const float up = WIDE ? 128.f : 1.f;
+            d = make_float4(up * rest(d.x), up * rest(d.y), up * rest(d.z), up * rest(d.w));
+          }
+        }
+      }
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncthreads();
+      if (tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x, buf ^ 1);
+      const bf16* xa = &sX[buf][((tap / 3) * WT + tap % 3 + (ln & 7) + (ln >> 4) * 8) * XS + ((ln >> 3) & 1) * 8];
+      const int ob = ((ln & 7) + ((ln >> 3) & 1) * 8) * XS + (ln >> 4) * 8;
+#pragma unroll
+      for (int ti = 0; ti < GH; ++ti) {
+        uint32_t a[2][4];
+        ldsm4t(a[0], xa + ti * WT * XS);
+        ldsm4t(a[1], xa + ti * WT * XS + 16);
+        auto lower = [&](uint32_t x) {   // X for the lower terms
+          return WIDE ? x & ~__vcmpeq2(x & 0x7fff7fffu, 0x7f807f80u) : x;
+        };
+#pragma unroll
+        for (int n2 = 0; n2 < 2; ++n2) {
+          float r[2][2][4];   // the sums over this row's 16 pixels
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) r[m][0][e] = r[m][1][e] = 0.f;
+#pragma unroll
+          for (int s = 2; s >= 0; --s) {   // the small terms first
+            uint32_t bq[4];
+            ldsm4t(bq, &sD[s][ti * TW * XS + ob + n2 * 16]);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              uint32_t x[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) x[e] = s > 0 ? lower(a[m][e]) : a[m][e];
+              mma_bf16(r[m][0], x[0], x[1], x[2], x[3], bq[0], bq[1]);
+              mma_bf16(r[m][1], x[0], x[1], x[2], x[3], bq[2], bq[3]);
+              if (WIDE && s > 0) {
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { r[m][0][e] = r[m][0][e] * 0.0078125f; r[m][1][e] = r[m][1][e] * 0.0078125f; }
+              }
+            }
+          }
+#pragma unroll
+          for (int m = 0; m < 2; ++m)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              acc[m][2 * n2][e] = acc[m][2 * n2][e] + r[m][0][e];
+              acc[m][2 * n2 + 1][e] = acc[m][2 * n2 + 1][e] + r[m][1][e];
+            }
         }
       }
     }
-    asm volatile("cp.async.wait_all;\n" ::: "memory");
-    __syncthreads();
-    if (tile + (int)gridDim.x < ntiles) fetch(tile + gridDim.x, buf ^ 1);
-    const bf16* xa = &sX[buf][((tap / 3) * WT + tap % 3 + (ln & 7) + (ln >> 4) * 8) * XS + ((ln >> 3) & 1) * 8];
-    const int ob = ((ln & 7) + ((ln >> 3) & 1) * 8) * XS + (ln >> 4) * 8;
+    bool met = least < (kTiny << 1) - 1u;
+    if (!WIDE)   // NaN: perhaps an infinite X against a zero term
 #pragma unroll
-    for (int ti = 0; ti < GH; ++ti) {
-      uint32_t a[2][4];
-      ldsm4t(a[0], xa + ti * WT * XS);
-      ldsm4t(a[1], xa + ti * WT * XS + 16);
+      for (int m = 0; m < 2; ++m)
 #pragma unroll
-      for (int n2 = 0; n2 < 2; ++n2) {
-        float r[2][2][4];   // the sums over this row's 16 pixels
+        for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) r[m][0][e] = r[m][1][e] = 0.f;
-#pragma unroll
-        for (int s = 2; s >= 0; --s) {   // the small terms first
-          uint32_t bq[4];
-          ldsm4t(bq, &sD[s][ti * TW * XS + ob + n2 * 16]);
-#pragma unroll
-          for (int m = 0; m < 2; ++m) {
-            mma_bf16(r[m][0], a[m][0], a[m][1], a[m][2], a[m][3], bq[0], bq[1]);
-            mma_bf16(r[m][1], a[m][0], a[m][1], a[m][2], a[m][3], bq[2], bq[3]);
-          }
-        }
-#pragma unroll
-        for (int m = 0; m < 2; ++m)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            acc[m][2 * n2][e] = acc[m][2 * n2][e] + r[m][0][e];
-            acc[m][2 * n2 + 1][e] = acc[m][2 * n2 + 1][e] + r[m][1][e];
-          }
-      }
-    }
-  }
+          for (int e = 0; e < 4; ++e) met = met || isnan(acc[m][n][e]);
+    return met;
+  };
+  if (__syncthreads_or(walk(std::false_type{}))) walk(std::true_type{});
   float* o = part + (size_t)blockIdx.x * BLK_SZ;
   const int g = ln >> 2, q = ln & 3;
 #pragma unroll
