@@ -864,13 +864,15 @@ __global__ void k_density_init(Dev d) {
 }
 
 // Batched two-right-hand-side Thomas solver (trid) for the C-ABI unit entry points, one thread per
-// system, element k of system s at k * nsys + s (layer-major, coalesced).  One reciprocal of the
-// pivot per layer serves its three quotients.  The forward sweep loads the next TU layers while it
+// system, element k of system s at k * nsys + s (layer-major, coalesced).  Three quotients a layer, as
+// the reference forms them: with one reciprocal of the pivot for the three a call was 1.6 us faster, but
+// the quotients were rounded twice (error 1.7e-16 instead of
+// 1.5e-16) and a pivot below 5.6e-309 overflowed.  The forward sweep loads the next TU layers while it
 // eliminates the current ones; with SHM it keeps the eliminated values in shared memory, so that a
 // call moves its five inputs and two outputs once, and otherwise in c1, ag and ar.  A few thousand
-// systems leave the chip mostly idle: the sweep's dependent chain (a reciprocal a layer) and the
-// first loads are the time.  40 layers x 20011 systems, synchronous call: 93 us with three divisions
-// and one layer's loads in flight, 30 us so (14 us of it the call itself).
+// systems leave the chip mostly idle: the sweep's dependent chain (a division a layer) and the
+// first loads are the time.  40 layers x 20011 systems, synchronous call: 93 us with one layer's loads
+// in flight, 29 us so (14 us of it the call itself).
 constexpr int TT = 32, TU = 4;
 template <bool SHM>
 __global__ void __launch_bounds__(TT) k_column_tridiag(int n, int nsys, const double* a, const double* b, const double* c,
@@ -903,10 +905,9 @@ __global__ void __launch_bounds__(TT) k_column_tridiag(int n, int nsys, const do
         gv = gv - v.a[u] * dp;
         rv = rv - v.a[u] * ep;
       }
-      const double q = 1.0 / den;
-      cp = v.c[u] * q;
-      dp = gv * q;
-      ep = rv * q;
+      cp = v.c[u] / den;
+      dp = gv / den;
+      ep = rv / den;
       if (SHM) {
         s_el[(3 * k) * TT + threadIdx.x] = cp;
         s_el[(3 * k + 1) * TT + threadIdx.x] = dp;
