@@ -24,8 +24,8 @@
 //           memory only.  A block publishes z as tagged words that carry their own arrival, like
 //           the barrier's slots; the neighbours form the halo's p = z + beta p themselves.  No
 //           fence is needed in the iteration.
-//   stream  for blocks whose window does not fit: z and p go through L2, with fences at the
-//           exchange that follows their writes.
+//   stream  for blocks whose window does not fit or whose halo is long: z and p go through L2, with fences
+//           at the exchange that follows their writes.
 //   cluster the window form for up to eight blocks: one thread-block cluster, whose blocks exchange
 //           sums and z through each other's shared memory, behind the cluster's barrier; a block has
 //           at most one node a thread, with its coefficients in registers.  3924 unknowns, four
@@ -68,12 +68,22 @@ __host__ __device__ constexpr long long window_bytes(int per, int reach) {
   return ((long long)per + 4LL * reach + 1 + 3) / 4 * 4 * (long long)sizeof(T);
 }
 // The window form runs when the window leaves room for at least a quarter of the block's nodes
-// (a block of 512 threads then still reads most of a phase's data from shared memory) and its
-// entries fit 16-bit indices.
+// (a block of 512 threads then still reads most of a phase's data from shared memory), its
+// entries fit 16-bit indices, and the halo is short: its words are polled one after the other by each
+// thread, some 1.5 us an iteration for every thousand nodes of reach, where the stream form pays for its
+// fences and for reading z and p of the eight neighbours through L2.  Basins that are long along the
+// numbering's fast index have a long reach.  Window / stream, us an iteration in FP64 and FP32 (the
+// latter with the refinement around it), by reach and nodes a block:
+//   1000,  500: 4.5 / 5.3 and 7.0 / 7.4     2000,  500: 6.7 / 5.7 and 9.0 / 7.7     2000, 640: 8.0 / 9.7, 10.5 / 10.0
+//   1500, 1440: 8.8 / 11.4, 11.2 / 12.5     2000, 3200: 19.9 / 22.7, 20.7 / 22.2
+//   4000,  500: 8.9 / 5.6 and 11.0 / 7.8    4000, 1280: 12.4 / 11.6, 14.7 / 10.9    4000, 2570: 18.8 / 18.6, 19.7 / 18.0
+//   8000,  770: - / 11.9 and 20.6 / 10.3
+// One block alone has no halo.
 template <typename T>
-__host__ __device__ inline bool window_fits(int per, int reach) {
+__host__ __device__ inline bool window_fits(int per, int nb, int reach) {
   const long long w = window_bytes<T>(per, reach);
-  return per + 2LL * reach + 1 < 65536 && w + (long long)node_bytes<T, true>() * (per / 4) <= kSmemMax;
+  const bool near = nb == 1 || (reach <= 3000 && 4LL * reach <= 13LL * per);
+  return near && per + 2LL * reach + 1 < 65536 && w + (long long)node_bytes<T, true>() * (per / 4) <= kSmemMax;
 }
 
 // z of one node as a tagged word: every 8-byte part carries the tag (coop.cuh's slots).
@@ -470,9 +480,9 @@ template <typename T>
 __device__ __forceinline__ void schur_any(const PcgDevT<T>& P, GridBar* bar, int bid, int nb, int smem) {
   const int per = (P.B.n + nb - 1) / nb;
   const long long all = window_bytes<T>(per, P.reach) + (long long)((per + 1) / 2 * 2) * node_bytes<T, true>();
-  if (per <= SB && all <= smem) schur_body<T, true, true>(P, bar, bid, nb, smem);
-  else if (window_fits<T>(per, P.reach)) schur_body<T, true, false>(P, bar, bid, nb, smem);
-  else schur_body<T, false, false>(P, bar, bid, nb, smem);
+  if (!window_fits<T>(per, nb, P.reach)) schur_body<T, false, false>(P, bar, bid, nb, smem);
+  else if (per <= SB && all <= smem) schur_body<T, true, true>(P, bar, bid, nb, smem);
+  else schur_body<T, true, false>(P, bar, bid, nb, smem);
 }
 
 template <typename T>
@@ -547,7 +557,7 @@ int launch_schur(const PcgDevT<T>& P, GridBar* bar, int nblocks, cudaStream_t st
   }
   const size_t pitch = sizeof(uint4) * (size_t)slot_plane(P.slot_blocks);
   if (cudaMemset2DAsync(P.slots, pitch, 0, sizeof(uint4) * (size_t)nblocks, 2 * kSlotVals, st) != cudaSuccess) return -1;
-  const int smem = (int)std::min<long long>(kSmemMax, window_fits<T>(per, P.reach) ? win : (long long)pe * node_bytes<T, false>());
+  const int smem = (int)std::min<long long>(kSmemMax, window_fits<T>(per, nblocks, P.reach) ? win : (long long)pe * node_bytes<T, false>());
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[1];
   coop_config(cfg, attr, nblocks, smem, st);
