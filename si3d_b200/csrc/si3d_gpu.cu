@@ -204,8 +204,10 @@ struct Ctx {
   // Zeroed device memory that lives as long as the handle.  Arrays up to kSlabItem bytes share slabs: a
   // handle has about a hundred of them, and an allocation with its zero fill and synchronisation (and
   // the free at the end) costs 0.1 to 0.2 ms each (the stand-alone zeta solve of 52500 columns, which
-  // makes and drops a handle: 34 ms with one allocation per array).
-  static constexpr size_t kSlabItem = 4 << 20, kSlab = 32 << 20;
+  // makes and drops a handle: 34 ms with one allocation per array).  A slab is about what the handle's
+  // arrays need, so that a small basin takes little memory.
+  static constexpr size_t kSlabItem = 4 << 20, kSlabMin = 2 << 20, kSlabMax = 32 << 20;
+  size_t slab_size = kSlabMax;
   char* slab = nullptr;
   size_t slab_left = 0;
   int fresh(void** q, size_t bytes) {
@@ -227,9 +229,10 @@ struct Ctx {
       if (int rc = fresh(&q, bytes)) return rc;
     } else {
       if (slab_left < bytes) {
-        if (int rc = fresh(&q, kSlab)) return rc;
+        const size_t size = std::max(slab_size, bytes);
+        if (int rc = fresh(&q, size)) return rc;
         slab = static_cast<char*>(q);
-        slab_left = kSlab;
+        slab_left = size;
       }
       q = slab;
       slab += bytes;
@@ -1342,6 +1345,12 @@ static int init_handle(const si3d_grid* g, const si3d_params* prm, int device, b
   c->lm = lm; c->lm1 = lm1; c->km1 = km1; c->P = P;
   Dev& d = c->d;
   d.g.lm = lm; d.g.lm1 = lm1; d.g.km1 = km1; d.g.km = km1 - 1; d.g.k1 = g->k1; d.g.P = P;
+  {
+    // about 600 bytes a column for maps, 2-D fields and the zeta system, and the 3-D fields that go in slabs
+    const size_t n3 = sizeof(double) * (size_t)km1 * P;
+    const size_t need = 600 * (size_t)P + (solver_only || n3 > Ctx::kSlabItem ? 0 : 36 * n3);
+    c->slab_size = std::min(std::max(need, Ctx::kSlabMin), Ctx::kSlabMax);
+  }
   int rc = 0;
   // maps, padded to P; the sentinel column lm1 points to itself
   auto up_int = [&](const int* src, int nsrc, int fill) -> const int* {
