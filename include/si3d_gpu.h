@@ -320,9 +320,10 @@ int si3d_ens_nodes(int ens);
 /* How the captured step runs the members' zeta solves (no counterpart in the reference).
  * SI3D_ENS_SOLVE_BATCHED (the default): the members advance in lock step, and each of the step's
  * zeta solves is ONE cooperative launch for all members, each basin iterating to its own
- * convergence on its share of the SMs with its own barrier counter; it applies when every member
+ * convergence on its share of the SMs with its own barrier record; it applies when every member
  * uses stopping test 5, the same itrap and niter, and no open boundary, and there are no more
- * members than co-resident blocks (otherwise the step falls back to the per-member form).
+ * members than co-resident blocks (otherwise the step falls back to the per-member form).  A pond
+ * of less than 32 columns of one colour solves by a launch of its own beside that one.
  * SI3D_ENS_SOLVE_MEMBERS: one cooperative solve launch per member, on the member's own stream.
  * A member that gets as many blocks in the batched launch as its own launch uses (the members'
  * needs fit the GPU together) sums its dot products in the same order, and both forms give

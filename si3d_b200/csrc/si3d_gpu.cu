@@ -2142,16 +2142,17 @@ struct Ens {
   size_t nodes = 0;
   std::vector<cudaEvent_t> joins;
   cudaEvent_t fork = nullptr, t0 = nullptr, t1 = nullptr, solved = nullptr;
-  // batched solves: every zeta solve of the step is one cooperative launch for all members
-  int mode = SI3D_ENS_SOLVE_BATCHED;   // requested; the per-member form when a member does not qualify
+  // batched solves: every zeta solve of the step is one cooperative launch for the members in `batch`
+  int mode = SI3D_ENS_SOLVE_BATCHED;   // requested; the per-member form when the step does not qualify
   bool batched = false;                // the form of the captured graph
   int loop_blocks = 0;                 // blocks of the batched launch
   int slots = 0;                       // batched launches per step (zeta solves of a step)
-  std::vector<double> nodes_of;        // nodes of each member's larger colour
-  std::vector<int> caps;               // blocks of each member's own solve launch
-  PcgEnsItem* d_items = nullptr;       // [slots][members] shares of the batched launches
+  std::vector<int> batch;              // members whose solves are batched (the others launch their own)
+  std::vector<double> nodes_of;        // black nodes of each of these
+  std::vector<int> caps;               // blocks of each one's own solve launch
+  PcgEnsItem* d_items = nullptr;       // [slots][batch] shares of the batched launches
   GridBar* d_bars = nullptr;
-  uint4* d_slots = nullptr;            // barrier slots of all members, one after the other
+  uint4* d_slots = nullptr;            // barrier slots of all of these, one after the other
   size_t slot_n = 0;
   ~Ens() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -2197,42 +2198,47 @@ int si3d_ens_create(const int* handles, int n, int* ens) {
   return 0;
 }
 
-// Whether every member qualifies for the batched solves: stopping test 5, no stored diagonal, no
-// recording, the same time-stepping options, and no more members than co-resident blocks.  Fixes
+// Whether the step qualifies for the batched solves: stopping test 5, no stored diagonal, no
+// recording and the same time-stepping options for every member, and no more members in the batch than
+// co-resident blocks.  The batch is the members that are solved on the black unknowns; the others (a
+// pond of a few columns) solve by a launch of their own on their own stream beside it.  Fixes
 // the launch's grid (every co-resident block, or the sum of the members' own launch sizes if
 // smaller) and the solves a step has.
 static bool ens_batch_plan(Ens* E) {
   const int m = (int)E->hs.size();
   const si3d_params& p0 = get(E->hs[0])->prm;
-  E->nodes_of.assign(m, 0.0);
-  E->caps.assign(m, 1);
+  E->batch.clear();
+  E->nodes_of.clear();
+  E->caps.clear();
   long long own = 0;
   for (int i = 0; i < m; ++i) {
     const Ctx* c = get(E->hs[i]);
-    if (!c->pcg.cf || c->pcg.diag_stored || c->rec_buf || c->prm.itrap != p0.itrap ||
-        c->prm.niter != p0.niter || c->schur_blk < 1)
+    if (c->prm.pcg_test != 5 || c->pcg.diag_stored || c->rec_buf || c->prm.itrap != p0.itrap ||
+        c->prm.niter != p0.niter)
       return false;
-    E->nodes_of[i] = c->pcg.B.n;
-    E->caps[i] = c->schur_blk;
+    if (!c->pcg.cf) continue;
+    E->batch.push_back(i);
+    E->nodes_of.push_back(c->pcg.B.n);
+    E->caps.push_back(c->schur_blk);
     own += c->schur_blk;
   }
   const int nb = pcg_loop_ens_blocks(E->device);
-  if (nb < m) return false;
+  if (E->batch.empty() || nb < (int)E->batch.size()) return false;
   E->loop_blocks = (int)std::min<long long>(nb, own);
   const bool leapfrog_only = p0.itrap == 0 || (2 % std::max(p0.itrap, 1)) != 0;
   E->slots = leapfrog_only ? 1 : 1 + std::min(p0.niter, 21);
   return true;
 }
 
-// The members' shares of one batched launch, for solves that took its[i] iterations (all 1 before
+// The shares of the batch in one launch, for solves that took its[member] iterations (all 1 before
 // any step): one block each, then one more at a time to the member whose solve would take longest,
-// its[i] x (a fixed cost per iteration + its nodes per block x a streaming cost per node), up to the
-// blocks its own launch uses (its partial-sum arrays are sized for those).  Every block of the grid
+// iterations x (a fixed cost per iteration + its nodes per block x a streaming cost per node), up to the
+// blocks its own launch uses (its barrier slots are sized for those).  Every block of the grid
 // is given out.
 static std::vector<int> ens_shares(const Ens* E, const std::vector<double>& its) {
   constexpr double kIterUs = 2.9;      // the two exchanges of an iteration
   constexpr double kNodeUs = 0.0026;   // one black node (1183 a block: 5.9 us an iteration, 491: 4.1 us)
-  const int m = (int)E->hs.size();
+  const int m = (int)E->batch.size();
   std::vector<int> b(m, 1);
   int left = E->loop_blocks - m;
   while (left > 0) {
@@ -2240,7 +2246,7 @@ static std::vector<int> ens_shares(const Ens* E, const std::vector<double>& its)
     double bv = -1.0;
     for (int i = 0; i < m; ++i) {
       if (b[i] >= E->caps[i]) continue;
-      const double t = its[i] * (kIterUs + kNodeUs * E->nodes_of[i] / b[i]);
+      const double t = its[E->batch[i]] * (kIterUs + kNodeUs * E->nodes_of[i] / b[i]);
       if (t > bv) { bv = t; best = i; }
     }
     if (best < 0) break;
@@ -2253,16 +2259,16 @@ static std::vector<int> ens_shares(const Ens* E, const std::vector<double>& its)
 // Upload the shares of every solve slot of the step (its: [slot][member] iterations, or null for
 // the first plan).
 static int ens_upload_shares(Ens* E, const std::vector<std::vector<double>>* its) {
-  const int m = (int)E->hs.size();
+  const int m = (int)E->batch.size();
   std::vector<PcgEnsItem> items((size_t)m * E->slots);
   std::vector<size_t> at(m + 1, 0);
   for (int i = 0; i < m; ++i) at[i + 1] = at[i] + schur_slots(E->caps[i]);
   for (int k = 0; k < E->slots; ++k) {
-    const std::vector<int> b = ens_shares(E, its ? (*its)[k] : std::vector<double>(m, 1.0));
+    const std::vector<int> b = ens_shares(E, its ? (*its)[k] : std::vector<double>(E->hs.size(), 1.0));
     int first = 0;
     for (int i = 0; i < m; ++i) {
       PcgEnsItem& it = items[(size_t)k * m + i];
-      it.P = get(E->hs[i])->pcg;
+      it.P = get(E->hs[E->batch[i]])->pcg;
       it.P.slots = E->d_slots + at[i];
       it.bar = E->d_bars + i;
       it.first = first;
@@ -2277,14 +2283,17 @@ static int ens_upload_shares(Ens* E, const std::vector<std::vector<double>>* its
 // Capture one step (n >= 2) with every zeta solve batched: the members advance in lock step on their
 // own streams up to each solve's set-up, join the master stream for one cooperative launch that
 // solves all of their systems (k_schur_loop_ens, each member on its share of the blocks with its own
-// barrier record), and fork again for the rest of the fd call.  The stage sequence is step_impl's
+// barrier record), and fork again for the rest of the fd call; members outside the batch run their own
+// solve launches on their own streams.  The stage sequence is step_impl's
 // for n >= 2.  The k-th launch reads its shares from slot k of the item array, which the steps
 // refresh from each solve's last iteration counts without capturing again.
 static int ens_capture_batched(Ens* E) {
-  const int m = (int)E->hs.size();
+  const int m = (int)E->hs.size(), nbatch = (int)E->batch.size();
+  std::vector<char> batched(m, 0);
+  for (int i : E->batch) batched[i] = 1;
   if (!E->d_items) {
-    CK(cudaMalloc(&E->d_bars, sizeof(GridBar) * (size_t)m));
-    CK(cudaMalloc(&E->d_items, sizeof(PcgEnsItem) * (size_t)m * E->slots));
+    CK(cudaMalloc(&E->d_bars, sizeof(GridBar) * (size_t)nbatch));
+    CK(cudaMalloc(&E->d_items, sizeof(PcgEnsItem) * (size_t)nbatch * E->slots));
     for (int cap : E->caps) E->slot_n += schur_slots(cap);
     CK(cudaMalloc(&E->d_slots, sizeof(uint4) * E->slot_n));
     const int rc = ens_upload_shares(E, nullptr);
@@ -2299,7 +2308,7 @@ static int ens_capture_batched(Ens* E) {
     Ctx* c = cs[i] = get(E->hs[i]);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(c->st, E->fork, 0);
     c->graph_mode = true;
-    c->ens_defer = true;
+    c->ens_defer = batched[i] != 0;
     c->solve_slot = 0;
     c->trap_solves = 0;
     c->thrs = 2.0 * c->prm.dt / 3600.;
@@ -2314,20 +2323,24 @@ static int ens_capture_batched(Ens* E) {
       int r = fd_pre(cs[i], istep);
       if (!r) r = solve(cs[i], &it, &rr, &ie);
       if (r) return r;
+      if (!batched[i]) continue;
       if (cudaEventRecord(E->joins[i], cs[i]->st) != cudaSuccess ||
           cudaStreamWaitEvent(E->master, E->joins[i], 0) != cudaSuccess)
         return cuda_fail(cudaGetLastError());
     }
     if (slot >= E->slots) return SI3D_EDIMS;
-    if (pcg_loop_ens(E->d_items + (size_t)slot * m, m, E->loop_blocks, E->d_bars, E->d_slots,
+    if (pcg_loop_ens(E->d_items + (size_t)slot * nbatch, nbatch, E->loop_blocks, E->d_bars, E->d_slots,
                      sizeof(uint4) * E->slot_n, E->master) != 0)
       return cuda_fail(cudaGetLastError(), "pcg_loop_ens", __LINE__);
     ++slot;
     cs[0]->launches += 1;
     if (cudaEventRecord(E->solved, E->master) != cudaSuccess) return cuda_fail(cudaGetLastError());
     for (int i = 0; i < m; ++i) {
-      if (cudaStreamWaitEvent(cs[i]->st, E->solved, 0) != cudaSuccess) return cuda_fail(cudaGetLastError());
-      int r = solve_graph_post(cs[i], cs[i]->def_hist, cs[i]->def_ier);
+      int r = 0;
+      if (batched[i]) {
+        if (cudaStreamWaitEvent(cs[i]->st, E->solved, 0) != cudaSuccess) return cuda_fail(cudaGetLastError());
+        r = solve_graph_post(cs[i], cs[i]->def_hist, cs[i]->def_ier);
+      }
       if (!r) r = fd_post(cs[i], last);
       if (r) return r;
     }
