@@ -713,12 +713,12 @@ int momentum_init(int km1) {
 }
 
 template <int IEQ>
-void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu, cudaStream_t st,
-                const ObcDev* obc, int nobc) {
+int launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu, cudaStream_t st,
+               const ObcDev* obc, int nobc) {
   if (tu.mom_cl == 1 && nobc == 0) {   // one pass per column (open boundaries need the split kernels)
     k_mom_fused<IEQ><<<tiles.ntile, MT, kMomSmem, st>>>(d, cols, tiles);
     k_mom_back<IEQ, BT><<<(d.g.lm + BT - 1) / BT, BT, 0, st>>>(d);
-    return;
+    return 2;
   }
   const int g1 = (ncols + CW - 1) / CW;
   switch (tu.mom_cl) {
@@ -727,21 +727,24 @@ void launch_dir(const Dev& d, const FaceMeta* cols, int ncols, const MomTiles& t
     default: k_mom_cells<IEQ, 8><<<g1, dim3(CW, 8), 0, st>>>(d, cols, ncols); break;
   }
   // open boundaries: MODexmom4openBCX/Y replace the explicit term of their face columns
-  for (int b = 0; b < nobc; ++b) obc_exmom(d, obc[b], IEQ, st);
+  int n = 3;
+  for (int b = 0; b < nobc; ++b) n += obc_exmom(d, obc[b], IEQ, st);
   switch (tu.mom_nt) {
     case 64: k_mom_columns<IEQ, 64><<<(ncols + 63) / 64, 64, 0, st>>>(d, cols, ncols); break;
     case 256: k_mom_columns<IEQ, 256><<<(ncols + 255) / 256, 256, 0, st>>>(d, cols, ncols); break;
     default: k_mom_columns<IEQ, 128><<<(ncols + 127) / 128, 128, 0, st>>>(d, cols, ncols); break;
   }
   k_mom_back<IEQ, BT><<<(d.g.lm + BT - 1) / BT, BT, 0, st>>>(d);
+  return n;
 }
 
-void launch_momentum(const Dev& d, int ieq, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu,
-                     cudaStream_t st, const ObcDev* obc, int nobc) {
+int launch_momentum(const Dev& d, int ieq, const FaceMeta* cols, int ncols, const MomTiles& tiles, const Tune& tu,
+                    cudaStream_t st, const ObcDev* obc, int nobc) {
   if (ieq == 1) k_mom_rho<BT><<<(d.g.lm + BT - 1) / BT, BT, 0, st>>>(d);   // both directions' sums
-  if (ncols <= 0) return;
-  if (ieq == 1) launch_dir<1>(d, cols, ncols, tiles, tu, st, obc, nobc);
-  else launch_dir<2>(d, cols, ncols, tiles, tu, st, obc, nobc);
+  const int rho = ieq == 1 ? 1 : 0;
+  if (ncols <= 0) return rho;
+  return rho + (ieq == 1 ? launch_dir<1>(d, cols, ncols, tiles, tu, st, obc, nobc)
+                         : launch_dir<2>(d, cols, ncols, tiles, tu, st, obc, nobc));
 }
 
 }  // namespace si3d

@@ -147,11 +147,12 @@ void obc_set_s(const Dev& d, const ObcDev& B, double v, cudaStream_t st) {
   if (B.n > 0) k_obc_set_s<<<grid(B.n), OB, 0, st>>>(d, B.cells, B.n, v);
 }
 
-void obc_exmom(const Dev& d, const ObcDev& B, int ieq, cudaStream_t st) {
+int obc_exmom(const Dev& d, const ObcDev& B, int ieq, cudaStream_t st) {
   const bool x = B.side == 1 || B.side == 3;
-  if ((ieq == 1) != x || B.nface <= 0) return;
+  if ((ieq == 1) != x || B.nface <= 0) return 0;
   const int kind = B.side == 1 ? 0 : B.side == 3 ? 1 : B.side == 2 ? 2 : 3;
   k_obc_exmom<<<grid(B.nface), OB, 0, st>>>(d, B.mom, B.nface, kind);
+  return 1;
 }
 
 void obc_qq(const Dev& d, const ObcDev& B, cudaStream_t st) {

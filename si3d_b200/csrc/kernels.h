@@ -82,9 +82,9 @@ int momentum_init(int km1);
 int transport_init(int km1);
 struct ObcDev;
 // `obc` (nobc boundaries): open boundaries whose face columns' explicit term is recomputed between
-// the cell and the column kernels
-void launch_momentum(const Dev& d, int ieq, const FaceMeta* meta, int ncols, const MomTiles& tiles, const Tune& tu,
-                     cudaStream_t st, const ObcDev* obc = nullptr, int nobc = 0);
+// the cell and the column kernels.  Returns the number of kernels launched.
+int launch_momentum(const Dev& d, int ieq, const FaceMeta* meta, int ncols, const MomTiles& tiles, const Tune& tu,
+                    cudaStream_t st, const ObcDev* obc = nullptr, int nobc = 0);
 void launch_matcon(const Dev& d, cudaStream_t st);
 
 void pcg_setup(const Dev& d, const PcgDev& P, int x0_mode, const double* dz, const double* hist, int* negpiv,
@@ -147,7 +147,7 @@ struct ObcDev {
   const int* mom = nullptr;
 };
 void obc_set_s(const Dev& d, const ObcDev& B, double v, cudaStream_t st);
-void obc_exmom(const Dev& d, const ObcDev& B, int ieq, cudaStream_t st);
+int obc_exmom(const Dev& d, const ObcDev& B, int ieq, cudaStream_t st);
 void obc_qq(const Dev& d, const ObcDev& B, cudaStream_t st);
 void obc_vel(const Dev& d, const ObcDev& B, cudaStream_t st);
 void obc_sca(const Dev& d, const ObcDev& B, double salbc, cudaStream_t st);

@@ -1179,9 +1179,10 @@ int obc_uvh(Ctx* c) {
 }
 
 // Stages with the open-boundary adjustments that follow their kernels.
-void momentum_stage(Ctx* c, int ieq) {
-  if (ieq == 1) launch_momentum(c->d, 1, c->mce, c->nce, c->tce, c->tune, c->st, c->obc.data(), (int)c->obc.size());
-  else launch_momentum(c->d, 2, c->mcn, c->ncn, c->tcn, c->tune, c->st, c->obc.data(), (int)c->obc.size());
+int momentum_stage(Ctx* c, int ieq) {   // the kernels launched
+  if (ieq == 1)
+    return launch_momentum(c->d, 1, c->mce, c->nce, c->tce, c->tune, c->st, c->obc.data(), (int)c->obc.size());
+  return launch_momentum(c->d, 2, c->mcn, c->ncn, c->tcn, c->tune, c->st, c->obc.data(), (int)c->obc.size());
 }
 void matcon_stage(Ctx* c) {
   launch_matcon(c->d, c->st);
@@ -1219,8 +1220,8 @@ int fd_pre(Ctx* c, int istep) {
   if (rc) return rc;
   c->launches += obc_launches(c);
   // surfbc CASE(0) is a constant per-column wind set by the host (uair/vair/cdw fields)
-  rc = stage(c, ST_MOMX, 4 + obc_launches(c), [&] { momentum_stage(c, 1); });
-  if (!rc) rc = stage(c, ST_MOMY, 3 + obc_launches(c), [&] { momentum_stage(c, 2); });
+  rc = stage(c, ST_MOMX, 0, [&] { c->launches += momentum_stage(c, 1); });
+  if (!rc) rc = stage(c, ST_MOMY, 0, [&] { c->launches += momentum_stage(c, 2); });
   if (!rc) rc = stage(c, ST_MATCON, 1 + 2 * obc_launches(c), [&] { matcon_stage(c); });
   return rc;
 }
