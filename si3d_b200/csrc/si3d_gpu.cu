@@ -1524,6 +1524,10 @@ static int init_handle(const si3d_grid* g, const si3d_params* prm, int device, b
     // 75 / 81 us, 800 tiles 195 / 166 us, 1260 tiles 442 / 340 us)
     // and the scalar kernels with as many lanes as fill the chip (31 tiles 8 lanes 28, 4 lanes 30 us;
     // 800 tiles 79 and 69 us)
+    // Columns numbered without regard to the grid: neighbouring faces share no pairs of columns and the tiles
+    // stay half empty.  Split / fused: 121 faces a tile (row by row) 92 / 80 and 272 / 184 us, 42 faces
+    // (shuffled) 155 / 166 and 754 / 929 us; the tiles are full or nearly so for grids of any shape
+    if (c->nce + c->ncn < kMomFaces / 2 * (c->tce.ntile + c->tcn.ntile)) c->tune.mom_cl = 8;
     if (c->tce.ntile < sms) { c->tune.mom_cl = 8; c->tune.mom_nt = 64; c->tune.sal_cl = 8; c->tune.sal_nt = 128; }
   }
   }
