@@ -7,8 +7,9 @@
 // producer, MMA and epilogue warps; see there).  The data gradient for training is an implicit GEMM
 // on 8 x 16 pixel tiles with mma.sync m16n8k16 (M = 16 pixels of a tile row, N = 8 channels, K = 16
 // channels of one tap; 9 taps x 2 channel halves = 18 K-steps) with tap-flipped, channel-transposed
-// weights.  BF16 operands, FP32 accumulation.  The 4 -> 32 stem, the 32 -> 1 head and the weight
-// gradients are small and run on the FP32 cores, accumulating in a fixed order.
+// weights.  BF16 operands, FP32 accumulation.  The 32 -> 32 weight gradients run on the tensor cores too
+// (k_wgrad32: mma.sync on an exact split of the FP32 operand).  The 4 -> 32 stem, the 32 -> 1 head and
+// their weight gradients are small and run on the FP32 cores, accumulating in a fixed order.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cudaTypedefs.h>

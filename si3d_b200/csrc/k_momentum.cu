@@ -704,8 +704,7 @@ __global__ void __launch_bounds__(MT, 4) k_mom_fused(Dev d, const FaceMeta* __re
 
 }  // namespace
 
-int momentum_init(int km1) {
-  (void)km1;   // the fused kernel's ring does not depend on the column depth
+int momentum_init() {   // (the fused kernel's ring does not depend on the column depth)
   if (cudaFuncSetAttribute(k_mom_fused<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMomSmem) != cudaSuccess ||
       cudaFuncSetAttribute(k_mom_fused<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, kMomSmem) != cudaSuccess)
     return -1;

@@ -49,8 +49,8 @@ namespace {
 
 using namespace coop;
 
-constexpr int SB = 512;    // threads per block (one block per SM); fixed, so that a basin's sums do
-                           // not depend on the launch it is solved in
+constexpr int SB = 512;    // threads per block (one block per SM), in every launch: a basin's sums depend on
+                           // the number of its blocks alone
 constexpr int RN = 3;      // nodes of a thread whose vectors are in registers (1536 of a block)
 constexpr int kSmemMax = 225 * 1024;
 constexpr int kClusterMax = 8;   // blocks of a cluster (the portable limit)
@@ -586,8 +586,7 @@ int schur_init() {
 }
 
 // One block per SM at most, and no block with fewer nodes than threads.
-int schur_blocks(int device, int nB, int max_per_sm) {
-  (void)max_per_sm;
+int schur_blocks(int device, int nB) {
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   return std::max(1, std::min(sms, (nB + SB - 1) / SB));

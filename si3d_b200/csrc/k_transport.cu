@@ -866,13 +866,13 @@ __global__ void k_density_init(Dev d) {
 // Batched two-right-hand-side Thomas solver (trid) for the C-ABI unit entry points, one thread per
 // system, element k of system s at k * nsys + s (layer-major, coalesced).  Three quotients a layer, as
 // the reference forms them: with one reciprocal of the pivot for the three a call was 1.6 us faster, but
-// the quotients were rounded twice (error 1.7e-16 instead of
-// 1.5e-16) and a pivot below 5.6e-309 overflowed.  The forward sweep loads the next TU layers while it
-// eliminates the current ones; with SHM it keeps the eliminated values in shared memory, so that a
-// call moves its five inputs and two outputs once, and otherwise in c1, ag and ar.  A few thousand
-// systems leave the chip mostly idle: the sweep's dependent chain (a division a layer) and the
-// first loads are the time.  40 layers x 20011 systems, synchronous call: 93 us with one layer's loads
-// in flight, 29 us so (14 us of it the call itself).
+// the quotients were rounded twice (error 1.7e-16 instead of 1.5e-16) and a pivot below 5.6e-309
+// overflowed.  The forward sweep loads the next TU layers while it eliminates the current ones; with
+// SHM it keeps the eliminated values in shared memory, so that a call moves its five inputs and two
+// outputs once, and otherwise in c1, ag and ar.  A few thousand systems leave the chip mostly idle: the
+// sweep's dependent chain (a division a layer) and the first loads are the time.  40 layers x 20011
+// systems, synchronous call: 93 us with one layer's loads in flight, 29 us so (14 us of it the call
+// itself).
 constexpr int TT = 32, TU = 4;
 template <bool SHM>
 __global__ void __launch_bounds__(TT) k_column_tridiag(int n, int nsys, const double* a, const double* b, const double* c,
@@ -948,7 +948,7 @@ __global__ void __launch_bounds__(TT) k_column_tridiag(int n, int nsys, const do
 
 static inline int grid_of(int n) { return (n + TB - 1) / TB; }
 
-constexpr int BK_LANES = 4;   // layer lanes of the copy kernels (slayer_h, vel_uv, vel2)
+constexpr int BK_LANES = 4;   // layer lanes of the copy kernels (full slayer_h, vel2)
 constexpr int HALF_LANES = 2;   // layer lanes of k_half_level and k_save
 constexpr int CONT_LANES = 8;   // layer lanes of the continuity kernels (4 and 16 measured slower)
 // From this many columns on one thread per column fills the chip and the lanes' shared-memory planes only

@@ -77,7 +77,7 @@ struct MomTiles {
   int ntile = 0;
 };
 
-int momentum_init(int km1);
+int momentum_init();
 // Raises the continuity kernels' shared-memory limit for columns deeper than 95 levels.
 int transport_init(int km1);
 struct ObcDev;
@@ -173,7 +173,7 @@ int pcg_loop_ens(const PcgEnsItem* items, int nitems, int nblocks, GridBar* bars
 // The test-5 loop on the black unknowns (k_pcg_schur.cu).  init: raises the kernels' shared-memory
 // limits; blocks: the launch's grid for nB black nodes; slots: uint4 entries its barriers need.
 int schur_init();
-int schur_blocks(int device, int nB, int max_per_sm);
+int schur_blocks(int device, int nB);
 size_t schur_slots(int nblocks);
 int schur_loop(const PcgDev& P, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init = nullptr);
 int schur_loop_f(const PcgDevF& F, GridBar* bar, int nblocks, cudaStream_t st, const GridBar* init = nullptr);

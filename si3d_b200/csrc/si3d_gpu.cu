@@ -703,7 +703,8 @@ int build_pcg(Ctx* c, const si3d_grid* g) {
       rc |= c->alloc(p, n1);
   }
   if (rc) return rc;
-  // SI3D_PCG_BLOCKS_PER_SM caps the resident blocks per SM of the cooperative solve (tuning)
+  // SI3D_PCG_BLOCKS_PER_SM caps the resident blocks per SM of the two-colour cooperative solve (tuning; the loop
+  // on the black unknowns has one block an SM at most)
   const char* bps = std::getenv("SI3D_PCG_BLOCKS_PER_SM");
   c->loop_blocks = pcg_loop_blocks(c->device, nR, nB, bps ? std::atoi(bps) : 0, false);
   c->loop_blocks_f = pcg_loop_blocks(c->device, nR, nB, bps ? std::atoi(bps) : 0, true);
@@ -738,7 +739,7 @@ int build_pcg(Ctx* c, const si3d_grid* g) {
       for (int m : {k.x, k.y, k.z, k.w})
         if (m < nB) P.reach = std::max(P.reach, std::abs(m - j));
   }
-  c->schur_blk = schur_blocks(c->device, nB, bps ? std::atoi(bps) : 0);
+  c->schur_blk = schur_blocks(c->device, nB);
   if (closes) {
     const size_t n = std::max(nB, 1);
     rc |= c->alloc(&P.nb8, 8 * n);
@@ -1453,7 +1454,7 @@ static int init_handle(const si3d_grid* g, const si3d_params* prm, int device, b
   rc |= c->alloc(&c->d_stats_ii, 48);
   rc |= c->alloc(&c->d_stats_rr, 24);
   if (!solver_only) {
-  if (!rc && momentum_init(km1) != 0) { g_last_cuda = "momentum kernel shared-memory attribute"; rc = SI3D_ECUDA; }
+  if (!rc && momentum_init() != 0) { g_last_cuda = "momentum kernel shared-memory attribute"; rc = SI3D_ECUDA; }
   if (!rc && transport_init(km1) != 0) { g_last_cuda = "continuity kernel shared-memory attribute"; rc = SI3D_ECUDA; }
   // pixel (i - 1) * jm1 + (j - 1) of every wet column in the (im1, jm1) image of the learned
   // initial guess (only when the maps describe a real grid)
